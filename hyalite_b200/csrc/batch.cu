@@ -30,6 +30,7 @@ namespace hy {
 
 static constexpr int LCG = LONG_G, LCR = LONG_R;      // long pairs and the int16x2 band
 static constexpr int ICG = MAIN_G32, ICR = MAIN_R32;  // int32 items
+static constexpr int BATCH_BAND_WARPS = 16;           // warps of a band block at most
 static constexpr uint32_t LONG_W_MAX = 4096;          // largest long-pair split allowed
 
 struct ClassLaunch {
@@ -170,7 +171,7 @@ __global__ void batch_profile_kernel(const BatchQuery *queries, const BatchCtl *
 // End positions of each ScoreEnd query's winner: block `slot` reruns the winner's item with
 // position tracking when the winner lives in this kernel's partition (int16x2 pair or int32 item).
 template <class A, int PK>
-__global__ void __launch_bounds__(1024) batch_band_kernel(const BandLaunch L) {
+__global__ void __launch_bounds__(32 * BATCH_BAND_WARPS) batch_band_kernel(const BandLaunch L) {
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t slot = blockIdx.x;
     if (slot >= L.ctl->n_queries) return;
@@ -678,7 +679,7 @@ hy_status batch_create(const hy_db *const *dbs, uint32_t n_dbs, uint32_t max_que
     const size_t band_pass = std::max({pass_bytes_of(al, WIN_G * WIN_R, pb16), pass_bytes_of(al, WIN_G * WIN_R, pb32),
                                        tab_row * WIN_G * WIN_R});
     if (st == HY_OK && (std::max({sm_bulk32, sm_long, sm_i32, sm_tbulk32, sm_tlong}) > (size_t)smem_optin ||
-                        128 + band_pass > (size_t)smem_optin)) {
+                        128 + band_smem_bytes(1, band_pass, WIN_R) > (size_t)smem_optin)) {
         st = fail(HY_ERR_UNSUPPORTED, al, smem_optin);
     }
     if (st == HY_OK) {
@@ -695,10 +696,11 @@ hy_status batch_create(const hy_db *const *dbs, uint32_t n_dbs, uint32_t max_que
         ck(prepare_class<Pair16, MAIN_G, 16, PK_BULK, true>(b, BC_SW16, sm_bulk16, n_sm));
         ck(prepare_class<PairTab16, MAIN_G, 8, PK_BULK, true>(b, BC_TSW8, sm_tbulk8, n_sm));
         ck(prepare_class<PairTab16, MAIN_G, 16, PK_BULK, true>(b, BC_TSW16, sm_tbulk16, n_sm));
-        int warps = (int)std::min<size_t>(32, BAND_SMEM_BUDGET / std::max<size_t>(band_pass, 1));
+        int warps = (int)std::min({(size_t)BATCH_BAND_WARPS, BAND_SMEM_BUDGET / std::max<size_t>(band_pass, 1),
+                                   ((size_t)smem_optin - 128 - band_smem_bytes(0, 0, WIN_R)) / (band_pass + band_warp_bytes(WIN_R))});
         warps = std::max(1, warps);
         b->band_threads = 32 * warps;
-        b->band_smem = 128 + (size_t)warps * band_pass;
+        b->band_smem = 128 + band_smem_bytes(warps, band_pass, WIN_R);
         ck(cudaFuncSetAttribute(batch_band_kernel<Pair16, PK_W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->band_smem));
         ck(cudaFuncSetAttribute(batch_band_kernel<Single32, PK_W32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->band_smem));
         ck(cudaFuncSetAttribute(batch_band_kernel<PairTab16, PK_W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->band_smem));

@@ -278,9 +278,9 @@ __global__ void winner_loc_kernel(const unsigned long long *key, const uint32_t 
 
 // The band kernel on one block, or on a cluster of `blocks` blocks (at most 8, the portable
 // cluster size every launch shape of one block per SM can be given).
-template <class A, int MODE, bool GPROF>
+template <class A, int R, int MODE, bool GPROF>
 static cudaError_t launch_band_mode(const ScanParams &p, int warps, int blocks, size_t smem, cudaStream_t st) {
-    auto kern = band_kernel<A, WIN_R, MODE, GPROF>;
+    auto kern = band_kernel<A, R, MODE, GPROF>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -312,12 +312,16 @@ struct BandShape {
     bool gprof;
     int warps, blocks;
     size_t smem;
+    int rows;  // rows per lane
 };
 static BandShape band_shape(const QueryPlan &qp, size_t smem_limit) {
     BandShape sh;
-    const size_t budget = std::min<size_t>(BAND_SMEM_BUDGET, smem_limit - 16);
+    const size_t budget = std::min<size_t>(BAND_SMEM_BUDGET, smem_limit - band_smem_bytes(1, 0, WIN_R));
+    sh.rows = WIN_R;
     sh.gprof = qp.pass_bytes > budget;
-    int warps = sh.gprof ? 32 : (int)std::min<size_t>(32, budget / std::max<uint32_t>(qp.pass_bytes, 1));
+    int warps = sh.gprof ? 32
+                         : (int)std::min({(size_t)32, budget / std::max<uint32_t>(qp.pass_bytes, 1),
+                                          (smem_limit - band_smem_bytes(0, 0, WIN_R)) / (qp.pass_bytes + band_warp_bytes(WIN_R))});
     warps = std::max(1, std::min(warps, std::max(qp.n_passes, 1)));
     int blocks = 1;
     if (!sh.gprof && qp.n_passes > warps) {
@@ -327,8 +331,42 @@ static BandShape band_shape(const QueryPlan &qp, size_t smem_limit) {
     }
     sh.warps = warps;
     sh.blocks = blocks;
-    sh.smem = sh.gprof ? 16 : (size_t)warps * qp.pass_bytes + 16;
+    sh.smem = band_smem_bytes(warps, sh.gprof ? 0 : qp.pass_bytes, WIN_R);
     return sh;
+}
+
+// The shape a band of lane arithmetic A runs a query of length qlen in, and its plan: 4 rows per lane
+// on blocks of 4 warps, so that a warp has its scheduler to itself, on up to 8 blocks of a cluster,
+// and more warps a block beyond that, while all passes fit one round of at most 16 warps a block;
+// else 8 rows per lane. (2000 x 2000 / 5000 x 5000 int32 pair: 0.231 / 0.674 ms; 2 warps a block 0.229
+// / 0.674, and 0.27 against 0.22 for 3 passes; 8 warps 0.268 / 0.712; 8 rows per lane 0.61 / 1.65.)
+template <class A>
+static BandShape band_plan(uint64_t qlen, uint64_t al, size_t smem_limit, QueryPlan &qp) {
+    qp = plan_for<A>(qlen, WIN_G * BAND_FEW_ROWS, al);
+    const int blocks = std::max(1, std::min(BAND_CLUSTER_MAX, (qp.n_passes + 3) / 4));
+    const int warps = std::max(1, (qp.n_passes + blocks - 1) / blocks);
+    const size_t smem = band_smem_bytes(warps, qp.pass_bytes, BAND_FEW_ROWS);
+    if (warps <= band_max_warps<BAND_FEW_ROWS>() && smem <= smem_limit) return {false, warps, blocks, smem, BAND_FEW_ROWS};
+    qp = plan_for<A>(qlen, WIN_G * WIN_R, al);
+    return band_shape(qp, smem_limit);
+}
+
+template <class A>
+static cudaError_t launch_band(int mode, const BandShape &sh, const ScanParams &p, cudaStream_t st) {
+#define HY_BAND_CASE(M)                                                                                     \
+    case M:                                                                                                 \
+        return sh.gprof             ? launch_band_mode<A, WIN_R, M, true>(p, sh.warps, 1, sh.smem, st)      \
+               : sh.rows == WIN_R   ? launch_band_mode<A, WIN_R, M, false>(p, sh.warps, sh.blocks, sh.smem, st) \
+                                    : launch_band_mode<A, BAND_FEW_ROWS, M, false>(p, sh.warps, sh.blocks, sh.smem, st);
+    switch (mode) {
+        HY_BAND_CASE(MODE_SW)
+        HY_BAND_CASE(MODE_NW)
+        HY_BAND_CASE(MODE_HW)
+        HY_BAND_CASE(MODE_OV)
+        HY_BAND_CASE(MODE_SHW)
+    }
+#undef HY_BAND_CASE
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace hy
@@ -352,9 +390,13 @@ static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &
                               uint32_t item_end, const uint8_t *d_query, uint64_t qlen,
                               uint8_t *prof, void *bnd, const uint32_t *item_ptr) {
     const bool i16 = A::NH == 2;
-    QueryPlan qp = plan_for<A>(qlen, WIN_G * WIN_R, db->al);
-    HY_CK((launch_profile<A, WIN_G, WIN_R>(db, d_query, qlen, qp, i16 ? lim16(db) : LIM32, prof,
-                                            sc->stream)));
+    QueryPlan qp;
+    const BandShape sh = band_plan<A>(qlen, db->al, db->smem_limit, qp);
+    const int32_t lim = i16 ? lim16(db) : LIM32;
+    if (sh.rows == WIN_R)
+        HY_CK((launch_profile<A, WIN_G, WIN_R>(db, d_query, qlen, qp, lim, prof, sc->stream)));
+    else
+        HY_CK((launch_profile<A, WIN_G, BAND_FEW_ROWS>(db, d_query, qlen, qp, lim, prof, sc->stream)));
     ScanParams p{};
     p.meta = part.d_meta;
     p.item_base = 0;
@@ -377,25 +419,7 @@ static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &
     p.err = sc->d_err;
     p.wait_polls = wait_polls();
     set_extents<A>(p, db, part, part.total_cols);
-    BandShape sh = band_shape(qp, db->smem_limit);
-    const bool gprof = sh.gprof;
-    const int warps = sh.warps, blocks = sh.blocks;
-    const size_t smem = sh.smem;
-    cudaError_t e = cudaErrorInvalidValue;
-#define HY_BAND_CASE(M)                                                                        \
-    case M:                                                                                    \
-        e = gprof ? launch_band_mode<A, M, true>(p, warps, 1, smem, sc->stream)                \
-                  : launch_band_mode<A, M, false>(p, warps, blocks, smem, sc->stream);         \
-        break;
-    switch (db->mode) {
-        HY_BAND_CASE(MODE_SW)
-        HY_BAND_CASE(MODE_NW)
-        HY_BAND_CASE(MODE_HW)
-        HY_BAND_CASE(MODE_OV)
-        HY_BAND_CASE(MODE_SHW)
-    }
-#undef HY_BAND_CASE
-    HY_CK(e);
+    HY_CK(launch_band<A>(db->mode, sh, p, sc->stream));
     sc->launches += qp.n_passes > 0 ? 2 : 1;
     return fail(HY_OK);
 }
@@ -482,9 +506,10 @@ static hy_status band_pair_enqueue(BandPairContext &c, const uint8_t *d_q, uint6
                                    const int32_t *d_matrix, uint64_t al, int32_t go, int32_t ge, int mode,
                                    cudaStream_t st, uint32_t slot, int32_t *d_scores, int32_t *d_qend,
                                    int32_t *d_tend) {
-    const QueryPlan qp = plan_for<Single32>(m, WIN_G * WIN_R, al);
+    QueryPlan qp;
+    const BandShape sh = band_plan<Single32>(m, al, c.smem_limit, qp);
     HY_CK(grow_dev(c.prof, c.c_prof, std::max<size_t>(16, (size_t)qp.pass_bytes * qp.n_passes)));
-    HY_CK(grow_dev(c.bnd, c.c_bnd, sizeof(int32_t) * std::max<uint64_t>(16, 2 * tl)));
+    HY_CK(grow_dev(c.bnd, c.c_bnd, sizeof(int32_t) * (2 * tl + 16)));
     // The item (the target as one int32 column run, the pair's slot as its index), its index and
     // a cleared error word.
     ItemMeta im{};
@@ -502,9 +527,11 @@ static hy_status band_pair_enqueue(BandPairContext &c, const uint8_t *d_q, uint6
     HY_CK(cudaMemcpyAsync(c.meta, c.h_stage, 40, cudaMemcpyHostToDevice, st));
     const uint8_t *base = reinterpret_cast<const uint8_t *>(c.meta);
     const bool top_free = mode == MODE_SW || mode == MODE_HW || mode == MODE_OV;
-    const int64_t words = Single32::letters((int64_t)al) * WIN_G * WIN_R * (int64_t)qp.n_passes;
+    const int64_t words = Single32::letters((int64_t)al) * WIN_G * sh.rows * (int64_t)qp.n_passes;
     if (words > 0) {
-        build_profile_kernel<Single32, WIN_G, WIN_R><<<(int)std::min<int64_t>((words + 255) / 256, 148 * 16), 256, 0, st>>>(
+        auto kern = sh.rows == WIN_R ? build_profile_kernel<Single32, WIN_G, WIN_R>
+                                     : build_profile_kernel<Single32, WIN_G, BAND_FEW_ROWS>;
+        kern<<<(int)std::min<int64_t>((words + 255) / 256, 148 * 16), 256, 0, st>>>(
             d_q, (int32_t)m, d_matrix, (int32_t)al, go, LIM32, top_free ? 1 : 0, qp.vrow0, qp.n_passes,
             reinterpret_cast<Single32::PE *>(c.prof));
         HY_CK(cudaGetLastError());
@@ -535,23 +562,8 @@ static hy_status band_pair_enqueue(BandPairContext &c, const uint8_t *d_q, uint6
     p.bnd_cols = tl;
     p.n_seqs = slot + 1;
     p.letters = (uint32_t)Single32::letters((int64_t)al);
-    const BandShape sh = band_shape(qp, c.smem_limit);
-    cudaError_t e = cudaErrorInvalidValue;
     HY_CK(cudaEventRecord(c.ev[0], st));
-#define HY_PAIR_BAND_CASE(M)                                                                      \
-    case M:                                                                                       \
-        e = sh.gprof ? launch_band_mode<Single32, M, true>(p, sh.warps, 1, sh.smem, st)           \
-                     : launch_band_mode<Single32, M, false>(p, sh.warps, sh.blocks, sh.smem, st); \
-        break;
-    switch (mode) {
-        HY_PAIR_BAND_CASE(MODE_SW)
-        HY_PAIR_BAND_CASE(MODE_NW)
-        HY_PAIR_BAND_CASE(MODE_HW)
-        HY_PAIR_BAND_CASE(MODE_OV)
-        HY_PAIR_BAND_CASE(MODE_SHW)
-    }
-#undef HY_PAIR_BAND_CASE
-    HY_CK(e);
+    HY_CK(launch_band<Single32>(mode, sh, p, st));
     HY_CK(cudaEventRecord(c.ev[1], st));
     return fail(HY_OK);
 }
@@ -563,7 +575,7 @@ hy_status band_long_pair(const uint8_t *d_q, uint64_t m, const uint8_t *t, uint6
     hy_status s0 = band_pair_context(cp);
     if (s0 != HY_OK) return s0;
     BandPairContext &c = *cp;
-    HY_CK(grow_dev(c.in, c.c_in, std::max<uint64_t>(16, tl)));
+    HY_CK(grow_dev(c.in, c.c_in, tl + 16));
     if (tl) HY_CK(cudaMemcpyAsync(c.in, t, tl, cudaMemcpyHostToDevice, st));
     s0 = band_pair_enqueue(c, d_q, m, c.in, tl, d_matrix, al, go, ge, mode, st, slot, d_scores, d_qend, d_tend);
     if (s0 != HY_OK) return s0;
@@ -585,8 +597,9 @@ hy_status band_single_pair(const uint8_t *q, uint64_t m, const uint8_t *t, uint6
     hy_status s0 = band_pair_context(cp);
     if (s0 != HY_OK) return s0;
     BandPairContext &c = *cp;
-    // Query, target and matrix staged together for one copy (the matrix 4-byte aligned).
-    const uint64_t mat_off = (m + tl + 3) / 4 * 4, bytes = mat_off + sizeof(int32_t) * al * al;
+    // Matrix, target and query staged together for one copy (the target's columns are read in
+    // pairs: on an even address, and one past the end).
+    const uint64_t t_at = sizeof(int32_t) * al * al, q_at = t_at + (tl + 15) / 16 * 16, bytes = q_at + m;
     if (bytes > c.ch_in) {
         if (c.h_in) cudaFreeHost(c.h_in);
         c.h_in = nullptr;
@@ -594,13 +607,13 @@ hy_status band_single_pair(const uint8_t *q, uint64_t m, const uint8_t *t, uint6
         HY_CK(cudaMallocHost((void **)&c.h_in, bytes));
         c.ch_in = bytes;
     }
-    memcpy(c.h_in, q, m);
-    memcpy(c.h_in + m, t, tl);
-    memcpy(c.h_in + mat_off, matrix, sizeof(int32_t) * al * al);
+    memcpy(c.h_in, matrix, t_at);
+    memcpy(c.h_in + t_at, t, tl);
+    memcpy(c.h_in + q_at, q, m);
     HY_CK(grow_dev(c.in, c.c_in, bytes));
     HY_CK(cudaMemcpyAsync(c.in, c.h_in, bytes, cudaMemcpyHostToDevice, c.stream));
     int32_t *d_res = reinterpret_cast<int32_t *>(reinterpret_cast<uint8_t *>(c.meta) + 40);
-    s0 = band_pair_enqueue(c, c.in, m, c.in + m, tl, reinterpret_cast<const int32_t *>(c.in + mat_off), al, go, ge,
+    s0 = band_pair_enqueue(c, c.in + q_at, m, c.in + t_at, tl, reinterpret_cast<const int32_t *>(c.in), al, go, ge,
                            mode, c.stream, 0, d_res, d_res + 1, d_res + 2);
     if (s0 != HY_OK) return s0;
     HY_CK(cudaMemcpyAsync(c.h_stage + 36, reinterpret_cast<const uint8_t *>(c.meta) + 36, 16, cudaMemcpyDeviceToHost,

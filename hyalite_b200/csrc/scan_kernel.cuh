@@ -89,7 +89,7 @@ struct ScanParams {
     uint64_t res_cols;  // columns of the residue array
     uint64_t bnd_cols;  // columns the boundary region holds, from bnd_col0
     uint32_t n_seqs;    // db indices are below this
-    uint32_t letters;   // profile letters per table
+    uint32_t letters;   // profile letters per table (the last is the padding symbol)
 };
 
 // Error words a kernel leaves in ScanParams::err: a bounded wait gave up, or (bounds-checked
@@ -160,6 +160,8 @@ struct Pair16 {
     __host__ __device__ static constexpr int64_t letters(int64_t al) { return al + 1; }
     // Residue code of a pair column (low sequence's symbol lo, high sequence's hi).
     __host__ __device__ static constexpr uint32_t code(uint32_t lo, uint32_t hi, uint32_t) { return lo | (hi << 8); }
+    // The padding column's residue code, of a profile of `letters` letters.
+    __host__ __device__ static constexpr uint32_t pad_code(uint32_t letters) { return (letters - 1) * 0x101u; }
 };
 
 // The int16x2 arithmetic with a half-size query profile, for kernels whose groups each keep their
@@ -199,6 +201,7 @@ struct PairTab16 : Pair16 {
     __host__ __device__ static constexpr uint32_t code(uint32_t lo, uint32_t hi, uint32_t al) {
         return lo * (al + 1) + hi;
     }
+    __host__ __device__ static constexpr uint32_t pad_code(uint32_t letters) { return letters - 1; }
     __device__ __forceinline__ static V diag(V g, V p, V) { return __vadd2(g, p); }
     __device__ __forceinline__ static void residues(RES r, int &a, int &b) {
         a = r;
@@ -260,6 +263,7 @@ struct Single32 {
     __host__ __device__ __forceinline__ static PE word(int64_t v, int) { return (PE)v; }
     static constexpr bool PAIRTAB = false;
     __host__ __device__ static constexpr int64_t letters(int64_t al) { return al + 1; }
+    __host__ __device__ static constexpr uint32_t pad_code(uint32_t letters) { return letters - 1; }
 };
 
 // Profile bytes per (letter, query row) of one lane arithmetic: every table's word.
@@ -392,12 +396,37 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(const void *p, int rank) {
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
-// The block barrier of a cluster of one, else the cluster barrier.
-__device__ __forceinline__ void band_sync(const int csize) {
-    if (csize > 1)
-        cluster_barrier();
-    else
-        __syncthreads();
+// The address of `p` in the shared memory of block `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, int rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+// 16 bytes to another block's shared memory, counted by an mbarrier there (both cluster addresses).
+__device__ __forceinline__ void st_async_v4(uint32_t dst, const uint4 v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait on an mbarrier that another block of the cluster completes.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, uint32_t polls) {
+    for (uint32_t it = 0; it < polls; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, "
+            "1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
 }
 // Whether `v` holds in any block of the cluster (`v` block-uniform; every thread calls it).
 // `flag` is a shared word of this block; no block returns before every block has read the others'.
@@ -422,7 +451,7 @@ __device__ __forceinline__ unsigned long long hit_key(int32_t score, uint32_t id
 // F values of its last row at column j reach lane L+1 at step s+1. Lane 0 reads the row above the
 // pass from the boundary row (or the top border in the first pass); lane G-1 writes the pass's
 // last row to the boundary row unless this is the last pass. The state lives in a Sweep so a
-// pass can be run in windows of steps (the block-cooperative band kernel interleaves warps).
+// pass can be run in windows of steps.
 template <class A, int R>
 struct Sweep {
     typename A::V Gp[R], E[R];  // G (= H - go) of the previous column and E, per row slot
@@ -625,10 +654,9 @@ __device__ __forceinline__ void sweep_step(Sweep<A, R> &sw, const int s, const i
 // Steps [s_begin, s_end) of one lane. `w_min` is the smallest item width in the warp: steps in
 // [G-1, w_min) have every lane of the warp on a real column and skip the per-lane checks. All
 // bounds are warp-uniform.
-// With PREFETCH the unchecked steps load the next step's residue code and boundary-row values one
-// step ahead; only for callers whose boundary row was written by an earlier, completed pass (the
-// band kernel's warps read rows another warp is writing and keep their exact read timing).
-template <class A, int G, int R, int MODE, bool ENDS, bool PREFETCH = false, bool COLMAX = false>
+// The unchecked steps load the next step's residue code and boundary-row values one step ahead (the
+// boundary row was written by an earlier, completed pass).
+template <class A, int G, int R, int MODE, bool ENDS, bool COLMAX = false>
 __device__ __forceinline__ void sweep_run(Sweep<A, R> &sw, const int s_begin, const int s_end,
                                           const int w_min, const int lane, const int32_t w,
                                           const uint32_t (&n)[2],
@@ -651,7 +679,7 @@ __device__ __forceinline__ void sweep_run(Sweep<A, R> &sw, const int s_begin, co
         sweep_step<A, G, R, MODE, ENDS, true, false, COLMAX>(sw, s, lane, w, n, res, prof_a, prof_b, row0,
                                                              first_pass, last_pass, bnd, qlen, go, ge, k,
                                                              best, cand, 0, 0, 0, cmo);
-    if (PREFETCH && fast_lo < fast_hi) {
+    if (fast_lo < fast_hi) {
         typedef typename A::V V;
         // Every lane of the warp is inside its item in [fast_lo, fast_hi): the indices below
         // (step s - lane, clamped to the range) are real columns.
@@ -677,11 +705,6 @@ __device__ __forceinline__ void sweep_run(Sweep<A, R> &sw, const int s_begin, co
             g_cur = g_next;
             f_cur = f_next;
         }
-    } else {
-        for (int s = fast_lo; s < fast_hi; ++s)
-            sweep_step<A, G, R, MODE, ENDS, false, false, COLMAX>(sw, s, lane, w, n, res, prof_a, prof_b,
-                                                                  row0, first_pass, last_pass, bnd, qlen,
-                                                                  go, ge, k, best, cand, 0, 0, 0, cmo);
     }
     for (int s = max(fast_hi, head_end); s < s_end; ++s)
         sweep_step<A, G, R, MODE, ENDS, true, false, COLMAX>(sw, s, lane, w, n, res, prof_a, prof_b, row0,
@@ -714,7 +737,7 @@ __device__ __forceinline__ void sweep_pass(const int lane, const int steps, cons
     Sweep<A, R> sw;
     sweep_begin<A, R, MODE>(sw, row0, go, ge, Sv);
     if constexpr (COLMAX) sw.botM = A::splat(-(int64_t)go);
-    sweep_run<A, G, R, MODE, ENDS, true, COLMAX>(sw, 0, steps, w_min, lane, w, n, res, prof_a, prof_b,
+    sweep_run<A, G, R, MODE, ENDS, COLMAX>(sw, 0, steps, w_min, lane, w, n, res, prof_a, prof_b,
                                                  row0, first_pass, last_pass, bnd, qlen, go, ge, Sv,
                                                  best, cand, cmo);
     sweep_end<A, R, MODE, ENDS>(sw, row0, go, cand);
@@ -1231,31 +1254,261 @@ __global__ void __launch_bounds__(256, (scan_min_blocks<A, G, R, two_col_form<A,
     scan_unit<A, G, R, MODE, ENDS, GPROF>(p, first, end, smem, bars, phase);
 }
 
-// ---- the block-cooperative band kernel (one long item, with end positions) -------------------
+// ---- the block-cooperative band kernel (long items, with end positions) ----------------------
 //
-// Recovers the end positions of a single item (the winner of a scan) with a whole block. Every
-// warp is one 32-lane group running one pass (a band of 32*R query rows); the block takes the
-// passes in rounds of W = blockDim/32. Inside a round warp w runs BAND_K*2*w steps behind warp w-1
-// with a block barrier every BAND_K steps, so each boundary-row column a band reads was written
-// by the band above in an earlier window (the write of column j happens 2*BAND_K - (G - 1) >
-// BAND_K steps before the read). The round's profile slices are staged by one TMA bulk copy.
-constexpr int BAND_K = 32;
+// Runs one item (the winner of a scan, a long pair) on a whole block or thread-block cluster, with
+// position tracking. Every warp is one 32-lane group running one pass (a band of 32*R query rows),
+// two columns a step: lane L works columns 2(s - L) and 2(s - L) + 1 (from 0) at step s. The warps
+// take the passes in rounds of W * (blocks). Inside a round warp g runs BAND_LAG * g steps behind
+// the block's warp 0, with a block barrier every BAND_K steps: lane 31 of the warp above writes column
+// pair c at its step c + 31, and the window of steps [s0, s0 + BAND_K) here reads pairs s0 .. s0 +
+// BAND_K - 1, all written before the window's barrier since BAND_LAG >= BAND_K + 31. Between blocks
+// the last warp stores its row into the next block's ring (st.async, counted by an mbarrier per
+// BAND_K pairs there), which gives each ring block back once read; the blocks share no other step
+// (a cluster barrier a window took 2850 cycles of its 3400).
+//
+// What bounds it is one warp's step: a lone warp issues a chain of dependent instructions with
+// nothing beside it (one column of 4 rows a step with plain loads: 66 instructions, 250 cycles). So a
+// step has two columns whose chains are independent but for a row's lag, and as few other instructions
+// as it can: residue codes lie in a strip of shared memory that is refilled every 32 steps, the row
+// above in a ring there that the warp above writes (warp 0 fills its own a window at a time, from the
+// border or from the boundary row in global memory), both read at constant offsets; a step's codes are
+// loaded two steps and its profile words one step ahead. 88 instructions, 190 cycles for two columns
+// (230 across blocks): 2000 x 2000 int32 0.47 to 0.23 ms, 5000 x 5000 1.45 to 0.67 ms. Local mode takes the short row chain (sweep_step) and tracks the best cell
+// once a step: the columns' maximum against the running one, its place looked up only where that
+// improves.
+constexpr int BAND_K = 16;
+constexpr int BAND_LAG = 48;
+constexpr int BAND_RING = 64;  // column pairs a ring holds: at least the lag plus a window
+static_assert(BAND_LAG >= BAND_K + 31 && BAND_LAG % BAND_K == 0 && 32 % BAND_K == 0, "a window's row above must be written before it");
+static_assert(BAND_RING >= BAND_LAG + BAND_K && BAND_RING % BAND_K == 0, "the ring must hold every pair not yet read");
 
-// The band recovery of item `item` (a valid item of p.meta) by the whole block, or by every block
-// of a thread-block cluster: the cluster's warps take the passes in rounds of W * (blocks), block
-// b's warps the passes b * W .. b * W + W - 1 of a round, and a cluster barrier takes the place of
-// the block barrier between windows (it orders the boundary-row writes of one block's warps before
-// the next block's reads). `bar` is an initialised mbarrier whose next wait parity is `phase`; the
-// block's dynamic shared memory (`smem`) holds W = blockDim/32 pass slices. Every thread of every
-// block must call it. With GPROF (single blocks only) the warps read their pass slices from the
-// profile in global memory; `smem` and `bar` are then unused.
+// Where a step improves a lane's best cell, the form with 4 rows per lane copies the step's two
+// columns to shared memory (predicated stores, no branch: 0.425 to 0.350 ms for a 2000 x 2000 pair) and
+// finds the row in them after the sweep; the form with 8 rows finds it there and then.
+template <int R>
+__host__ __device__ constexpr bool band_copies() {
+    return R <= 4;
+}
+
+// Shared memory of a band warp besides its pass slice: its last row (G, F of both columns) by
+// column pair, the residue codes of 96 column pairs, and the lanes' copied columns (two halves). A
+// block has one more ring, for the row above warp 0.
+constexpr size_t BAND_RING_BYTES = BAND_RING * 16;
+__host__ __device__ constexpr size_t band_warp_bytes(int rows) {
+    return BAND_RING_BYTES + 96 * 4 + (rows <= 4 ? (size_t)2 * 2 * rows * 4 * 32 : 0);
+}
+
+// The block's mbarriers: the profile copy's, then per ring block (BAND_K pairs) one that counts the
+// bytes of the row above and one by which the next block gives its ring block back.
+constexpr int BAND_SLOTS = BAND_RING / BAND_K;
+constexpr int BAND_BARS = 1 + 2 * BAND_SLOTS;
+
+// Shared memory of a band block of `warps` warps with pass slices of `slice` bytes (0: in global
+// memory): the slices, the rings, the rest of the warps' bytes, the mbarrier.
+__host__ __device__ inline size_t band_smem_bytes(size_t warps, size_t slice, int rows) {
+    return warps * (slice + band_warp_bytes(rows)) + BAND_RING_BYTES + BAND_BARS * 8;
+}
+
+// A band lane's state: a Sweep's, with the last row of both columns.
+template <class A, int R>
+struct Band : Sweep<A, R> {
+    typename A::V botG1, botF1;
+};
+
+// The first of a lane's R rows whose G in half h is b, or R.
+template <class A, int R>
+__device__ __forceinline__ int band_row(const typename A::V (&col)[R], const int h, const int32_t b) {
+    int row = R;
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r)
+        if (A::get(col[r], h) == b) row = r;
+    return row;
+}
+
+// Local mode: the columns j and j + 1 (their G in g0, g1) raise the lane's running best to cm in
+// some halves. Either the best cell's id, or (band_copies) a copy of both columns in `copy`, the
+// lane's uint4s 32 apart, and j as the id.
+template <class A, int R>
+__device__ __forceinline__ void band_improve(Band<A, R> &sw, const typename A::V (&g0)[R], const typename A::V (&g1)[R],
+                                             const int32_t j, const typename A::V cm0, const typename A::V cm, uint4 *copy) {
+    if constexpr (band_copies<R>()) {
+#pragma unroll
+        for (int h = 0; h < A::NH; ++h) {
+            const uint32_t mask = A::NH == 1 ? 0xffffffffu : h ? 0xffff0000u : 0xffffu;
+            if (((uint32_t)cm ^ (uint32_t)sw.pbest) & mask) {
+#pragma unroll
+                for (int c = 0; c < R / 4; ++c) {
+                    copy[((2 * h) * (R / 4) + c) * 32] = make_uint4((uint32_t)g0[4 * c], (uint32_t)g0[4 * c + 1], (uint32_t)g0[4 * c + 2], (uint32_t)g0[4 * c + 3]);
+                    copy[((2 * h + 1) * (R / 4) + c) * 32] = make_uint4((uint32_t)g1[4 * c], (uint32_t)g1[4 * c + 1], (uint32_t)g1[4 * c + 2], (uint32_t)g1[4 * c + 3]);
+                }
+                (h ? sw.pid1 : sw.pid0) = j;
+            }
+        }
+        sw.pbest = cm;
+    } else if (cm != sw.pbest) {
+        // In the first column unless the second is higher.
+#pragma unroll
+        for (int h = 0; h < A::NH; ++h) {
+            const int32_t b = A::get(cm, h);
+            if (b != A::get(sw.pbest, h)) {
+                const bool first = b == A::get(cm0, h);
+                (h ? sw.pid1 : sw.pid0) = first ? j * R + band_row<A, R>(g0, h, b) : (j + 1) * R + band_row<A, R>(g1, h, b);
+            }
+        }
+        sw.pbest = cm;
+    }
+}
+
+// The lane's best cell of the pass as a candidate (see band_improve).
+template <class A, int R, int MODE>
+__device__ __forceinline__ void band_end(Band<A, R> &sw, const int32_t row0, const int32_t go, const uint4 *copy,
+                                         Cand (&cand)[2]) {
+    if constexpr (ModeFlags<MODE>::local && band_copies<R>()) {
+#pragma unroll
+        for (int h = 0; h < A::NH; ++h) {
+            int32_t &id = h ? sw.pid1 : sw.pid0;
+            if (id < 0) continue;
+            const int32_t b = A::get(sw.pbest, h);
+            typename A::V g[2][R];
+#pragma unroll
+            for (int col = 0; col < 2; ++col)
+#pragma unroll
+                for (int c = 0; c < R / 4; ++c) {
+                    const uint4 v = copy[((2 * h + col) * (R / 4) + c) * 32];
+                    g[col][4 * c] = v.x;
+                    g[col][4 * c + 1] = v.y;
+                    g[col][4 * c + 2] = v.z;
+                    g[col][4 * c + 3] = v.w;
+                }
+            const int r0 = band_row<A, R>(g[0], h, b);
+            id = r0 < R ? id * R + r0 : (id + 1) * R + band_row<A, R>(g[1], h, b);
+        }
+    }
+    sweep_end<A, R, MODE, true>(sw, row0, go, cand);
+}
+
+// Both columns j, j + 1 (1-based) of a step of one lane's R rows, the profile words and the row above
+// given, the second column one row behind the first in the instruction stream. `lastG`: the running
+// best of the last query row (modes that answer there, lane 31 of the last pass); columns past a
+// half's end are never considered, so its running best may run ahead of its candidate there. END:
+// one of the columns may be a half's last one (modes that answer there).
+template <class A, int R, int MODE, bool END>
+__device__ __forceinline__ void band_columns(Band<A, R> &sw, const int32_t j, const uint32_t (&n)[2],
+                                             const typename A::V (&pa)[2][R], const typename A::V (&pb)[2][R],
+                                             const int32_t row0, const bool last_lane, const typename A::V upG0, const typename A::V upF0,
+                                             const typename A::V upG1, const typename A::V upF1, const int32_t qlen,
+                                             const int32_t go, const SweepConst<A> &k, typename A::V &lastG,
+                                             Cand (&cand)[2], uint4 *copy) {
+    typedef typename A::V V;
+    typedef ModeFlags<MODE> Fl;
+    static_assert(R % 2 == 0, "rows are folded into the columns' maxima in twos");
+    V f0 = upF0, f1 = upF1, c0 = upG0, c1 = upG1, g0[R], g1[R], cm0 = sw.pbest, cm1 = k.neggo;
+#pragma unroll
+    for (int t = 0; t <= R; ++t) {
+#pragma unroll
+        for (int col = 0; col < 2; ++col) {
+            const int r = t - col;
+            if (r < 0 || r >= R) continue;
+            V &f = col ? f1 : f0, &chain = col ? c1 : c0;
+            V(&g)[R] = col ? g1 : g0;
+            // Column j's diagonal and left neighbours are the column before it; column j + 1's are j's.
+            const V left = col ? g0[r] : sw.Gp[r];
+            const V diag = r == 0 ? (col ? upG0 : sw.diag) : (col ? g0[r > 0 ? r - 1 : 0] : sw.Gp[r > 0 ? r - 1 : 0]);
+            sw.E[r] = A::addmax(sw.E[r], k.negge, left);
+            const V d = A::diag(diag, pa[col][r], pb[col][r]);
+            f = A::addmax(f, k.negge, chain);
+            if (Fl::local) {
+                const V x = A::vadd(A::vmax3_relu(d, sw.E[r], d), k.neggo);
+                chain = x;  // F of the next row from x: see sweep_step
+                g[r] = A::addmax(f, k.neggo, x);
+                if (r & 1) {
+                    if (col)
+                        cm1 = A::vmax3(cm1, g[r - 1], g[r]);
+                    else
+                        cm0 = A::vmax3(cm0, g[r - 1], g[r]);
+                }
+            } else {
+                chain = g[r] = A::vadd(A::vmax3(d, sw.E[r], f), k.neggo);
+            }
+        }
+    }
+    sw.diag = upG1;
+    sw.botG = g0[R - 1];
+    sw.botF = f0;
+    sw.botG1 = g1[R - 1];
+    sw.botF1 = f1;
+    if (Fl::local) {
+        band_improve<A, R>(sw, g0, g1, j, cm0, A::vmax(cm0, cm1), copy);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) sw.Gp[r] = g1[r];
+    if (Fl::last_row && last_lane) {
+        const V m = A::vmax3(lastG, sw.botG, sw.botG1);
+        if (m != lastG) {
+#pragma unroll
+            for (int h = 0; h < A::NH; ++h) {
+                const int32_t nh = (int32_t)n[h];
+                if (j <= nh) consider(cand[h], A::get(sw.botG, h) + go, j, qlen);
+                if (j + 1 <= nh) consider(cand[h], A::get(sw.botG1, h) + go, j + 1, qlen);
+            }
+            lastG = m;
+        }
+    }
+    if constexpr (END && (Fl::last_col || Fl::corner)) {
+#pragma unroll
+        for (int h = 0; h < A::NH; ++h)
+#pragma unroll
+            for (int col = 0; col < 2; ++col) {
+                if (j + col != (int32_t)n[h]) continue;
+                const V(&g)[R] = col ? g1 : g0;
+                if (Fl::corner) {
+                    if (last_lane) consider(cand[h], A::get(g[R - 1], h) + go, j + col, qlen);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r)
+                        if (row0 + r >= 1) consider(cand[h], A::get(g[r], h) + go, j + col, row0 + r);
+                }
+            }
+    }
+}
+
+// A band warp's profile words of one residue code: row r's in pa[r] (and pb[r], two tables).
+template <class A, int R>
+__device__ __forceinline__ void band_words(const uint8_t *prof, const uint8_t *prof_hi, const uint32_t code,
+                                           const int lane, typename A::V (&pa)[R], typename A::V (&pb)[R]) {
+    int a, b;
+    A::residues((typename A::RES)code, a, b);
+#pragma unroll
+    for (int c = 0; c < R / A::EPV; ++c) {
+        typename A::V qa[A::EPV], qb[A::EPV];
+        A::template load_chunk<R, 32>(prof, prof_hi, a, b, lane, c, qa, qb);
+#pragma unroll
+        for (int e = 0; e < A::EPV; ++e) {
+            pa[c * A::EPV + e] = qa[e];
+            pb[c * A::EPV + e] = qb[e];
+        }
+    }
+}
+
+// The sweep of item `item` (a valid item of p.meta) by the whole block, or by every block of a
+// thread-block cluster: block b's warps take the passes b * W .. b * W + W - 1 of a round. `bar` is
+// an initialised mbarrier whose next wait parity is `phase` (a cluster's blocks: BAND_BARS of them,
+// not yet used); the block's dynamic shared memory (`smem`) holds W = blockDim/32 pass slices and
+// what band_smem_bytes adds. Every thread of every block must call it. With GPROF (single blocks only) the warps read their pass slices from the
+// profile in global memory; `bar` is then unused and `smem` holds the rings and strips alone.
 template <class A, int R, int MODE, bool GPROF = false>
 __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t item, uint8_t *smem,
                                           uint64_t *bar, uint32_t &phase) {
     typedef typename A::V V;
+    typedef typename A::RES RES;
+    typedef ModeFlags<MODE> Fl;
     constexpr int G = 32;
     constexpr int RPP = G * R;
-    static_assert(BAND_K >= G, "the lag must cover the lane skew of a warp");
+    // The residue codes of a column pair as one load: two 16-bit or two 8-bit codes.
+    typedef typename TwoCodes<A>::W W2;
+    constexpr int CODE_BITS = TwoCodes<A>::BITS;
+    constexpr uint32_t CODE_MASK = (1u << CODE_BITS) - 1u;
     static_assert(R % A::EPV == 0, "rows per lane must fill whole profile vectors");
     const int W = blockDim.x / G;
     const int warp = threadIdx.x / G, lane = threadIdx.x % G;
@@ -1272,12 +1525,30 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     }
 #endif
     const int32_t w = (int32_t)meta.w;
-    const V Sv = A::splat(p.sentinel);
-    const typename A::RES *res = reinterpret_cast<const typename A::RES *>(p.res) + meta.col_off;
-    V *bnd = reinterpret_cast<V *>(p.boundary) + 2 * (meta.col_off - p.bnd_col0);
-    V best = A::splat(0);
+    const RES *res = reinterpret_cast<const RES *>(p.res) + meta.col_off;
+    const W2 *res2 = reinterpret_cast<const W2 *>(res);
+    uint4 *bnd = reinterpret_cast<uint4 *>(reinterpret_cast<uint2 *>(p.boundary) + (meta.col_off - p.bnd_col0));
+    // Ring `warp` holds the row above this warp (ring 0: filled by warp 0 itself), ring warp + 1
+    // this warp's last row.
+    uint8_t *rings = smem + (GPROF ? 0 : (size_t)W * p.pass_bytes);
+    uint4 *in = reinterpret_cast<uint4 *>(rings + (size_t)warp * BAND_RING_BYTES);
+    uint4 *out = in + BAND_RING;
+    uint8_t *own = rings + (size_t)(W + 1) * BAND_RING_BYTES + (size_t)warp * (band_warp_bytes(R) - BAND_RING_BYTES);
+    W2 *strip = reinterpret_cast<W2 *>(own);
+    uint4 *copy = reinterpret_cast<uint4 *>(own + 96 * 4) + lane;
+    SweepConst<A> k;
+    k.negge = A::splat(-(int64_t)p.ge);
+    k.neggo = A::splat(-(int64_t)p.go);
+    k.Sv = A::splat(p.sentinel);
+    k.top_free_g = k.neggo;
     Cand cand[2] = {{INT32_MIN, INT32_MAX, INT32_MAX}, {INT32_MIN, INT32_MAX, INT32_MAX}};
-    const int pass_steps = w + G - 1;
+    const int pairs = (w + 1) / 2;  // column pairs
+    const int pass_steps = pairs + G - 1;
+    // Between blocks: ring blocks of BAND_K pairs, those of one slot in turn.
+    uint64_t *full = bar + 1, *empty = full + BAND_SLOTS;
+    const int n_blk = (pairs + BAND_K - 1) / BAND_K;
+    uint32_t full_ph = 0, empty_ph = 0;  // per slot: parity of its next wait at the round's start
+    auto blk_bytes = [&](int blk) { return 16u * (uint32_t)min(BAND_K, pairs - blk * BAND_K); };
     const int rounds = (p.n_passes + WT - 1) / WT;
     for (int round = 0; round < rounds; ++round) {
         const int first = round * WT;
@@ -1293,6 +1564,8 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                 phase ^= 1u;
                 fail = __syncthreads_or(!ok);
             }
+            if (csize > 1 && threadIdx.x == 0 && crank > 0 && bcnt > 0 && w > 0)
+                for (int blk = 0; blk < min(BAND_SLOTS, n_blk); ++blk) mbar_expect(full + blk, blk_bytes(blk));
             if (cluster_any(fail, &s_flag, csize)) {
                 if (threadIdx.x == 0 && fail) wait_gave_up(p.err, bar, 1u, phase ^ 1u);  // the round's copy
                 return;
@@ -1300,24 +1573,188 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
         }
         const int pass = first + gw;
         const bool mine = gw < cnt && w > 0;
+        const bool first_pass = pass == 0, last_pass = pass == p.n_passes - 1;
+        const bool last_lane = last_pass && lane == G - 1;
+        // Where the row above warp 0 comes from and where a block's last row goes.
+        const bool from_block = warp == 0 && crank > 0;
+        const bool to_block = warp == W - 1 && gw + 1 < cnt;
+        const bool to_bnd = !last_pass && gw + 1 == cnt;  // the round's last row: for the next round
+        bool waits = true;                                // until a wait gives up
+        auto wait_cluster = [&](uint64_t *b, uint32_t parity) {
+            if (waits && !mbar_wait_cluster(b, parity & 1u, p.wait_polls)) {
+                waits = false;
+                atomicExch(p.err, ERR_WAIT);
+            }
+            waits = __all_sync(0xffffffffu, waits);
+        };
         const int32_t row0 = p.vrow0 + pass * RPP + lane * R;
         const uint8_t *prof = GPROF ? p.profile + (size_t)min(pass, p.n_passes - 1) * p.pass_bytes
                                     : smem + (size_t)warp * p.pass_bytes;
         const uint8_t *prof_hi = prof + (A::TABLES - 1) * (p.pass_bytes / A::TABLES);
-        Sweep<A, R> sw;
-        sweep_begin<A, R, MODE>(sw, row0, p.go, p.ge, Sv);
-        const int lag = 2 * BAND_K * gw;
-        const int total = pass_steps + 2 * BAND_K * (cnt - 1);
-        for (int t0 = 0; t0 < total; t0 += BAND_K) {
-            const int s0 = max(t0 - lag, 0), s1 = min(t0 + BAND_K - lag, pass_steps);
-            if (mine && s0 < s1)
-                sweep_run<A, G, R, MODE, true>(sw, s0, s1, w, lane, w, meta.n, res, prof, prof_hi, row0,
-                                               pass == 0, pass == p.n_passes - 1, bnd, p.qlen, p.go,
-                                               p.ge, Sv, best, cand);
-            band_sync(csize);
+        Band<A, R> sw;
+        sweep_begin<A, R, MODE>(sw, row0, p.go, p.ge, k.Sv);
+        sw.botG1 = sw.botF1 = sw.botG;
+        sw.pbest = k.neggo;  // H = 0: only a cell above the border's 0 is tracked
+        V lastG = A::splat(A::VMIN);
+        // Codes of column pair c >= 0. An odd item's last pair holds the padding symbol in its second
+        // column, whose cells never exceed a real one in local mode and are never considered in others.
+        const uint32_t pad = A::pad_code(p.letters);
+        auto code_at = [&](int c) -> W2 {
+            const uint32_t v = 2 * c < w ? (uint32_t)res2[c] : pad;
+            return (W2)(2 * c + 1 < w ? v : (v & CODE_MASK) | (pad << CODE_BITS));
+        };
+        // This lane's pair of the 32 pairs before the strip's base, from it on, and after those.
+        W2 c_prev = 0, c_cur = 0, c_next = 0;  // (0: a valid letter)
+        V pa[2][R], pb[2][R];  // profile words of the coming step
+        uint32_t code = 0;     // residue codes of the step after it
+        auto words = [&](const uint32_t cc, V (&a)[2][R], V (&b)[2][R]) {
+            band_words<A, R>(prof, prof_hi, cc & CODE_MASK, lane, a[0], b[0]);
+            band_words<A, R>(prof, prof_hi, cc >> CODE_BITS, lane, a[1], b[1]);
+        };
+        if (mine) {
+            c_cur = code_at(lane);
+            c_next = code_at(G + lane);
+            strip[lane] = 0;
+            strip[G + lane] = c_cur;
+            __syncwarp();
+            words(strip[G - lane], pa, pb);
+            code = strip[G + 1 - lane];
         }
-        if (mine) sweep_end<A, R, MODE, true>(sw, row0, p.go, cand);
-        __syncthreads();  // the slices may be restaged for the next round
+        // Step s = s0 + i of the window at s0: `up` the row above at lane 0's pair, `cp` the strip at
+        // this lane's pair of step s0, `op` the ring slot of lane 31's pair. EDGE: lanes may not have
+        // started, be done (the row above is not defined past the item), or be at a half's last column.
+        auto step = [&](auto EDGE, const int s0, const int i, const uint4 up, const W2 *cp, uint4 *op) {
+            V upG0 = __shfl_up_sync(0xffffffffu, sw.botG, 1, G);
+            V upF0 = __shfl_up_sync(0xffffffffu, sw.botF, 1, G);
+            V upG1 = __shfl_up_sync(0xffffffffu, sw.botG1, 1, G);
+            V upF1 = __shfl_up_sync(0xffffffffu, sw.botF1, 1, G);
+            if (lane == 0) {
+                upG0 = (V)up.x;
+                upF0 = (V)up.y;
+                upG1 = (V)up.z;
+                upF1 = (V)up.w;
+            }
+            V na[2][R], nb[2][R];
+            words(code, na, nb);
+            code = cp[i + 2];
+            constexpr bool edge = decltype(EDGE)::value;
+            const int c = s0 + i - lane;
+            if (!edge || (c >= 0 && c < pairs))
+                band_columns<A, R, MODE, edge>(sw, 2 * c + 1, meta.n, pa, pb, row0, last_lane, upG0, upF0, upG1, upF1,
+                                               p.qlen, p.go, k, lastG, cand, copy);
+            if (lane == G - 1)
+                *op = make_uint4((uint32_t)sw.botG, (uint32_t)sw.botF, (uint32_t)sw.botG1, (uint32_t)sw.botF1);
+#pragma unroll
+            for (int col = 0; col < 2; ++col)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    pa[col][r] = na[col][r];
+                    pb[col][r] = nb[col][r];
+                }
+        };
+        // Whether a half's last column lies among the window's (modes that answer there).
+        auto ends_in = [&](int s0) {
+            if (!Fl::last_col && !Fl::corner) return false;
+            bool in_window = false;
+#pragma unroll
+            for (int h = 0; h < A::NH; ++h) {
+                const int c = ((int)meta.n[h] - 1) >> 1;  // the pair of half h's last column
+                in_window |= c > s0 - G && c < s0 + BAND_K;
+            }
+            return in_window;
+        };
+        const int total = bcnt > 0 ? pass_steps + BAND_LAG * (bcnt - 1) : 0;
+        for (int t0 = 0; t0 < total; t0 += BAND_K) {
+            const int s0 = t0 - BAND_LAG * warp;
+            if (mine && s0 >= 0 && s0 < pass_steps) {
+                if (from_block) {
+                    // Block b - 1's last warp writes the row above: the ring block read a window ago
+                    // goes back to it, and the next one must have arrived.
+                    const int blk = s0 / BAND_K, old = blk - 1;
+                    if (old >= 0 && old + BAND_SLOTS < n_blk && lane == 0) {
+                        mbar_expect(full + old % BAND_SLOTS, blk_bytes(old + BAND_SLOTS));
+                        mbar_arrive_cluster(cluster_addr(empty + old % BAND_SLOTS, crank - 1));
+                    }
+                    if (blk < n_blk)
+                        wait_cluster(full + blk % BAND_SLOTS, (full_ph >> (blk % BAND_SLOTS)) + (uint32_t)(blk / BAND_SLOTS));
+                } else if (warp == 0 && lane < BAND_K) {
+                    // The row above of the window's pairs: the top border, or the boundary row that
+                    // the round before wrote.
+                    const int c = s0 + lane;
+                    uint4 v = make_uint4(0, 0, 0, 0);
+                    if (first_pass) {
+                        auto top = [&](int j) {
+                            return (uint32_t)(Fl::top_free ? k.top_free_g : A::splat(-gap_pen(p.go, p.ge, j) - p.go));
+                        };
+                        v = make_uint4(top(2 * c + 1), (uint32_t)k.Sv, top(2 * c + 2), (uint32_t)k.Sv);
+                    } else if (c < pairs) {
+                        v = __ldcg(bnd + c);
+                    }
+                    in[c % BAND_RING] = v;
+                }
+                __syncwarp();  // no lane reads the strip's old codes any more
+                if (s0 % G == 0) {
+                    strip[lane] = c_prev;
+                    strip[G + lane] = c_cur;
+                    strip[2 * G + lane] = c_next;
+                    c_prev = c_cur;
+                    c_cur = c_next;
+                    c_next = code_at(s0 + 2 * G + lane);
+                }
+                __syncwarp();
+                const uint4 *ip = in + s0 % BAND_RING;
+                const W2 *cp = strip + G + s0 % G - lane;
+                // Lane 31 is at pair s - 31: slots 1 .. K - 1 of the ring's block at s0 - 32, then slot
+                // 0 of the next block.
+                uint4 *op = out + (s0 + BAND_RING - G) % BAND_RING + 1;
+                uint4 *op_last = out + (s0 + BAND_RING - G + BAND_K) % BAND_RING;
+                uint4 up = ip[0];
+                auto window = [&](auto EDGE) {
+                    for (int i0 = 0; i0 < BAND_K; i0 += 4) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const uint4 next = ip[i + 1];
+                            step(EDGE, s0 + i0, i, up, cp, i == 3 && i0 == BAND_K - 4 ? op_last : op + i);
+                            up = next;
+                        }
+                        ip += 4;
+                        cp += 4;
+                        op += 4;
+                    }
+                };
+                if (s0 >= G && s0 + BAND_K <= pairs && !ends_in(s0))
+                    window(std::false_type());
+                else
+                    window(std::true_type());
+                if (to_bnd || to_block) {
+                    static_assert(G == 2 * BAND_K, "a window's last pair begins a ring block");
+                    __syncwarp();
+                    const int c = s0 - (G - 1) + lane;
+                    const bool has = lane < BAND_K && c >= 0 && c < pairs;
+                    if (to_bnd) {
+                        if (has) bnd[c] = out[c % BAND_RING];
+                    } else {
+                        // Pairs s0 - 31 .. s0 - 16, the last one the first of its ring block, whose
+                        // earlier pairs the next block must have read.
+                        const int blk = s0 / BAND_K - 1;
+                        if (blk >= BAND_SLOTS && blk < n_blk)
+                            wait_cluster(empty + blk % BAND_SLOTS,
+                                         (empty_ph >> (blk % BAND_SLOTS)) + (uint32_t)(blk / BAND_SLOTS - 1));
+                        if (has)
+                            st_async_v4(cluster_addr(in - (size_t)warp * BAND_RING + c % BAND_RING, crank + 1), out[c % BAND_RING],
+                                        cluster_addr(full + (c / BAND_K) % BAND_SLOTS, crank + 1));
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        for (int k2 = 0; k2 < BAND_SLOTS; ++k2) {
+            const int uses = n_blk > k2 ? (n_blk - k2 + BAND_SLOTS - 1) / BAND_SLOTS : 0;
+            full_ph ^= (uint32_t)(uses & 1) << k2;
+            empty_ph ^= (uint32_t)(max(uses - 1, 0) & 1) << k2;
+        }
+        if (mine) band_end<A, R, MODE>(sw, row0, p.go, copy, cand);
+        __syncthreads();  // the slices and rings may be refilled for the next round
     }
     // Reduce every lane's candidates: inside each warp, then across warps in shared memory.
     __shared__ Cand s_cand[32][2];
@@ -1334,7 +1771,10 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
         }
         if (lane == 0) s_cand[warp][h] = cand[h];
     }
-    band_sync(csize);  // every block's candidates are in its shared memory
+    if (csize > 1)
+        cluster_barrier();  // every block's candidates are in its shared memory
+    else
+        __syncthreads();
     if (threadIdx.x == 0 && crank == 0) {
         for (int h = 0; h < A::NH; ++h) {
             const uint32_t idx = meta.idx[h];
@@ -1366,15 +1806,22 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     if (csize > 1) cluster_barrier();  // block 0 has read every block's candidates
 }
 
+// Warps of a band block at most: 32 where a block holds as many slices as fit (8 rows per lane),
+// 16 (128 registers a thread, no spills) for the form with fewer rows per lane.
+template <int R>
+constexpr int band_max_warps() {
+    return R < 8 ? 16 : 32;
+}
+
 template <class A, int R, int MODE, bool GPROF = false>
-__global__ void __launch_bounds__(1024) band_kernel(const ScanParams p) {
+__global__ void __launch_bounds__(32 * band_max_warps<R>(), 1) band_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t item = *p.item_ptr;
     if (item == NO_INDEX || item >= p.n_items) return;  // the same for every thread of the block
     const int W = blockDim.x / 32;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (GPROF ? 0 : (size_t)W * p.pass_bytes));
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + band_smem_bytes(W, GPROF ? 0 : p.pass_bytes, R)) - BAND_BARS;
     if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
+        for (int i = 0; i < BAND_BARS; ++i) mbar_init(bar + i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
