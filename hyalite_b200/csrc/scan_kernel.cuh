@@ -1292,11 +1292,13 @@ __host__ __device__ constexpr bool band_copies() {
 }
 
 // Shared memory of a band warp besides its pass slice: its last row (G, F of both columns) by
-// column pair, the residue codes of 96 column pairs, and the lanes' copied columns (two halves). A
+// column pair, the residue codes of 66 column pairs (32 before a block of 32 steps, 32 in it, and the
+// two loaded ahead), and the lanes' copied columns (two halves). A
 // block has one more ring, for the row above warp 0.
 constexpr size_t BAND_RING_BYTES = BAND_RING * 16;
+constexpr size_t BAND_STRIP_BYTES = (66 * 4 + 15) / 16 * 16;
 __host__ __device__ constexpr size_t band_warp_bytes(int rows) {
-    return BAND_RING_BYTES + 96 * 4 + (rows <= 4 ? (size_t)2 * 2 * rows * 4 * 32 : 0);
+    return BAND_RING_BYTES + BAND_STRIP_BYTES + (rows <= 4 ? (size_t)2 * 2 * rows * 4 * 32 : 0);
 }
 
 // The block's mbarriers: the profile copy's, then per ring block (BAND_K pairs) one that counts the
@@ -1535,7 +1537,7 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     uint4 *out = in + BAND_RING;
     uint8_t *own = rings + (size_t)(W + 1) * BAND_RING_BYTES + (size_t)warp * (band_warp_bytes(R) - BAND_RING_BYTES);
     W2 *strip = reinterpret_cast<W2 *>(own);
-    uint4 *copy = reinterpret_cast<uint4 *>(own + 96 * 4) + lane;
+    uint4 *copy = reinterpret_cast<uint4 *>(own + BAND_STRIP_BYTES) + lane;
     SweepConst<A> k;
     k.negge = A::splat(-(int64_t)p.ge);
     k.neggo = A::splat(-(int64_t)p.go);
@@ -1696,7 +1698,7 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                 if (s0 % G == 0) {
                     strip[lane] = c_prev;
                     strip[G + lane] = c_cur;
-                    strip[2 * G + lane] = c_next;
+                    if (lane < 2) strip[2 * G + lane] = c_next;
                     c_prev = c_cur;
                     c_cur = c_next;
                     c_next = code_at(s0 + 2 * G + lane);
