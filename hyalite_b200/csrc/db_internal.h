@@ -31,12 +31,13 @@ constexpr uint32_t LONG_W = 4096;
 constexpr uint32_t NO_LONG_SPLIT = 0xffffffffu;
 constexpr int BLOCK = 256;
 // Rows per lane of the bulk int16x2 kernel for a query of length qlen (passes of MAIN_G * rows).
-// SW scores run the two-column sweep at 8 or 16 rows per lane: 16 unless 8 pads the query to so
+// SW runs the two-column sweep at 8 or 16 rows per lane: 16 unless 8 pads the query to so
 // many fewer rows that it wins at 8 rows' rate per padded row (measured 0.853 of 16 rows' rate,
 // 4813 against 5641 GCUPS for 1000-residue queries on the protein benchmark: 150 residues take 192
 // rows at 8 against 256 at 16). The other kinds run one column of up to 32 rows.
-inline int bulk_rows(uint64_t qlen, bool two_col) {
+inline int bulk_rows(uint64_t qlen, bool two_col, bool ends = false) {
     if (qlen <= 64) return 8;
+    if (two_col && ends) return 16;  // the two-column sweep tracks ends from 12 rows per lane on
     if (two_col) {
         const uint64_t rows8 = (qlen + 63) / 64 * 64, rows16 = (qlen + 127) / 128 * 128;
         return 7 * rows8 < 6 * rows16 ? 8 : 16;
@@ -44,6 +45,7 @@ inline int bulk_rows(uint64_t qlen, bool two_col) {
     return qlen <= 192 ? 16 : 32;
 }
 constexpr int BULK_MAX_RPP = 8 * 32;
+constexpr int WIDE_MAX_RPP = 32 * 16;
 constexpr size_t BAND_SMEM_BUDGET = 200 * 1024;
 // Blocks of one band-kernel cluster at most (the portable cluster size).
 constexpr int BAND_CLUSTER_MAX = 8;
@@ -184,6 +186,146 @@ inline QuerySplit split_for_query(const hy_db *db, uint64_t qlen, uint32_t long_
     }
     q.kl = a;
     return q;
+}
+
+// Which pairs of a scan leave the bulk kernel for forms that finish one item sooner, and the int32
+// items' form (host only, from lengths alone). An item is one serial chain: in the bulk kernel on 8
+// lanes; in the wide form a warp (16 lanes for queries of at most 64 residues), a quarter of the
+// chain; in the band kernel a warp for every 128 query rows. The forms that finish sooner spend more
+// instructions a cell, so the split is the one of least estimated time. 50,000 protein sequences, best
+// hit with ends: a query of 350 residues 5.7 to 1.7 ms, of 5000 30.1 to 20.6; every target's ends, 500:
+// 10.7 to 2.9.
+struct ScanForms {
+    uint32_t band_end = 0;  // pairs [k0, band_end): the band kernel
+    uint32_t wide_end = 0;  // pairs [band_end, wide_end): the wide form; [wide_end, n): the bulk kernel
+    int wide_g = 32, wide_r = 8;
+    bool band32 = false;  // the int32 items: the band kernel, else a warp each
+};
+
+// Lanes and rows per lane of the wide form: one pass of the fewest rows up to 512 rows, longer queries
+// in passes of 512 or 256 rows by padded rows at their rates (8 rows 0.853 of 16 rows').
+inline void wide_shape(uint64_t qlen, bool two_col, int *g, int *r) {
+    *g = qlen <= 64 ? 16 : 32;
+    if (qlen <= 128) *r = 4;
+    else if (qlen <= 256) *r = 8;
+    else if (qlen <= 384 && two_col) *r = 12;
+    else if (qlen <= 512) *r = 16;
+    else *r = 7 * ((qlen + 255) / 256 * 256) < 6 * ((qlen + 511) / 512 * 512) ? 8 : 16;
+}
+
+// What the estimate is made of, fitted to measured kernels: a warp's instructions a step (one step of
+// two columns of r rows: 292 for 16 rows, 171 for 8; one column 9 a row, 13 with ends; the band's 100),
+// cycles an instruction of a scheduler with 4 warps (1.46) and of a lone warp (2.2), and what one more
+// kernel and its query profile take (cycles).
+struct ScanCost {
+    int mode;
+    bool ends;
+    // Instructions of one item's chain: passes of g * r rows over w columns.
+    double chain(uint64_t qlen, int g, int r, double w) const {
+        const double passes = (double)((qlen + (uint64_t)(g * r) - 1) / (uint64_t)(g * r));
+        if (mode == MODE_SW && scan_two_col_rows(r, ends)) return (passes * w / 2 + g) * ((ends ? 110.0 : 50.0) + 15.1 * r);
+        return passes * (w + g) * (50.0 + (mode == MODE_SW ? 13.0 : 9.0) * r);
+    }
+};
+constexpr double COST_SCHEDULERS = 148 * 4, COST_BUSY = 1.46, COST_ALONE = 2.2, COST_FORM = 16000;
+inline double band_chain(uint64_t qlen, double w) {
+    return (w / 2 + 51 + 48 * (double)((qlen - 1) / 128)) * 100;
+}
+// A band's warps hold their places for the whole chain, two or three to a scheduler (shared memory),
+// busy or not: 134 to 152 busy-rate instructions a step measured (72 items of 40 passes, 1093 of 3).
+inline double band_work(uint64_t qlen, double w) { return (double)((qlen + 127) / 128) * band_chain(qlen, w) * 1.5; }
+
+// Estimated cycles of `work` warp-instructions: the chip at its busy rate, then what is left of the
+// bulk's longest chain alone (`warps` bulk warps; `full`: the chain behind one warp a scheduler). The
+// other forms start first and their warps, the oldest of a scheduler, run nearly as if alone beside the
+// bulk: the longest of those bounds it, at 2.35 cycles an instruction (int32 chains of 12.1 M took 14.5
+// ms) or, a warp a pair, at 3.0 (blocks of 8 warps) or 3.7 (of 16: 4.0 M took 7.5 ms).
+struct ScanLoad {
+    double work = 0, bulk_warps = 0, bulk_chain = 0, full = 0, side_warps = 0, side_chain = 0, forms = 0;  // side_chain: cycles
+    double time() const {
+        const double busy = work / COST_SCHEDULERS * COST_BUSY;
+        const double rate = std::max(COST_ALONE, COST_BUSY * std::min(4.0, (bulk_warps + side_warps) / COST_SCHEDULERS));
+        const double bulk = std::max(busy, full * COST_ALONE) + std::max(0.0, bulk_chain - std::max(busy / rate, full)) * COST_ALONE;
+        const double side = side_chain * std::max(1.0, COST_BUSY / 2.35 * std::min(4.0, side_warps / COST_SCHEDULERS));
+        return std::max(bulk, side) + forms * COST_FORM;
+    }
+};
+
+inline ScanForms scan_forms(const hy_db *db, const QuerySplit &split, uint64_t qlen, bool ends, int bulk_r,
+                            int wide_g, int wide_r, int wide_threads) {
+    ScanForms f;
+    f.wide_g = wide_g;
+    f.wide_r = wide_r;
+    const ScanCost cost{db->mode, ends};
+    const uint32_t k0 = split.k0, n = db->p16.n_items;
+    f.band_end = f.wide_end = k0;
+    if (qlen == 0 || (k0 >= n && split.n_i32 == 0)) return f;
+    auto width = [&](uint32_t i) { return i < n ? (double)db->pair_w[i] : 0.0; };
+    auto mean = [&](uint32_t a, uint32_t b) {  // mean columns of pairs [a, b)
+        return b > a ? (double)(db->p16.res_prefix[b] - db->p16.res_prefix[a]) / 2 / (b - a) : 0.0;
+    };
+    // The int32 items: chains and work of both forms (their widths are the longest pairs').
+    const double w32 = split.n_i32 ? width(0) : 0.0, mean32 = mean(0, (split.n_i32 + 1) / 2);
+    auto time = [&](uint32_t band, uint32_t wide, bool band32) {
+        ScanLoad l;
+        auto side = [&](double count, double lanes, double each, double longest, double rate) {
+            if (count <= 0) return;
+            l.work += count * each * lanes / 32;
+            l.side_warps += count * lanes / 32;
+            l.side_chain = std::max(l.side_chain, longest * rate);
+            l.forms += 1;
+        };
+        if (band32) side(split.n_i32, 32, band_work(qlen, mean32), band_chain(qlen, w32), 2.35);
+        else side(split.n_i32, 32, cost.chain(qlen, 32, MAIN_R32, mean32), cost.chain(qlen, 32, MAIN_R32, w32), 2.35);
+        side(band - k0, 32, band_work(qlen, mean(k0, band)), band_chain(qlen, width(k0)), 2.35);
+        side(wide - band, f.wide_g, cost.chain(qlen, f.wide_g, f.wide_r, mean(band, wide)),
+             cost.chain(qlen, f.wide_g, f.wide_r, width(band)), wide_threads > BLOCK ? 3.7 : 3.0);
+        if (wide < n) {
+            const double count = n - wide;
+            l.work += count * cost.chain(qlen, MAIN_G, bulk_r, mean(wide, n)) * MAIN_G / 32;
+            l.bulk_warps = count * MAIN_G / 32;
+            l.bulk_chain = cost.chain(qlen, MAIN_G, bulk_r, width(wide));
+            const uint32_t i = wide + (uint32_t)COST_SCHEDULERS * (32 / MAIN_G);
+            if (i < n) l.full = cost.chain(qlen, MAIN_G, bulk_r, width(i));
+            l.forms += 1;
+        }
+        return l.time();
+    };
+    // Candidate splits: none, then pairs longer than 0.8^i of the longest, then all.
+    uint32_t cand[24];
+    int n_cand = 0;
+    double w = width(k0);
+    for (cand[n_cand++] = k0; n_cand < 23 && k0 < n; ++n_cand) {
+        w *= 0.8;
+        cand[n_cand] = (uint32_t)(std::partition_point(db->pair_w.begin() + k0, db->pair_w.end(),
+                                                       [&](uint32_t x) { return (double)x > w; }) -
+                                  db->pair_w.begin());
+    }
+    cand[n_cand++] = n;
+    double best = time(k0, k0, false);
+    // The int32 items' form, then the wide split, then the band split under it, then the wide one again.
+    if (split.n_i32) {
+        const double t = time(k0, k0, true);
+        if (t < best) best = t, f.band32 = true;
+    }
+    for (int round = 0; round < 2; ++round) {
+        for (int i = 0; i < n_cand; ++i) {
+            if (cand[i] < f.band_end) continue;
+            const double t = time(f.band_end, cand[i], f.band32);
+            if (t < best) best = t, f.wide_end = cand[i];
+        }
+        if (round == 0)
+            for (int i = 0; i < n_cand; ++i) {
+                const double t = time(cand[i], std::max(cand[i], f.wide_end), f.band32);
+                if (t < best) best = t, f.band_end = cand[i];
+            }
+        f.wide_end = std::max(f.wide_end, f.band_end);
+    }
+    if (split.n_i32) {
+        const double t = time(f.band_end, f.wide_end, !f.band32);
+        if (t < best) f.band32 = !f.band32;
+    }
+    return f;
 }
 
 }  // namespace hy

@@ -21,12 +21,13 @@ struct hy_scratch {
     const hy_db *db = nullptr;
     int device = 0;  // copied from the database: destroying a scratch never reads its database
     cudaStream_t stream = nullptr;
-    // The int32 part of a scan runs on a second stream, forked from and joined back into `stream`.
-    cudaStream_t stream2 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // The int32 items and the band items of a scan run on a second stream, the pairs a warp each on a
+    // third, forked from and joined back into `stream`.
+    cudaStream_t stream2 = nullptr, stream3 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
 
     uint8_t *d_query = nullptr;
-    uint8_t *d_prof16 = nullptr, *d_prof32 = nullptr, *d_profw16 = nullptr, *d_profw32 = nullptr;
+    uint8_t *d_prof16 = nullptr, *d_prof32 = nullptr, *d_profw16 = nullptr, *d_profw32 = nullptr, *d_profx16 = nullptr;
     void *d_bnd16 = nullptr, *d_bnd32 = nullptr;
     int32_t *d_scores = nullptr, *d_qend = nullptr, *d_tend = nullptr;
     unsigned long long *d_key = nullptr;
@@ -183,7 +184,7 @@ static hy_status enqueue_partition(const hy_db *db, hy_scratch *sc, const Partit
     p.err = sc->d_err;
     p.wait_polls = wait_polls();
     set_extents<A>(p, db, part, part.total_cols);
-    size_t smem = 2 * (size_t)qp.pass_bytes + 16;
+    size_t smem = scan_slices(qp.n_passes) * (size_t)qp.pass_bytes + scan_extra_smem(A::NH, R, db->mode, ends, threads);
     const bool gprof = smem > db->smem_limit;
     if (gprof) smem = 16;
     const bool timed = sc->profile && item_ptr == nullptr;
@@ -195,7 +196,7 @@ static hy_status enqueue_partition(const hy_db *db, hy_scratch *sc, const Partit
             sc->events.push_back({a, b});
             sc->event_part.push_back(0);
         }
-        const int cls = i16 ? 0 : 1;
+        const int cls = !i16 ? 1 : G == MAIN_G ? 0 : 2;
         sc->event_part[sc->n_events] = cls;
         sc->event_cells[cls] +=
             (double)qlen * (double)(part.res_prefix[item_end] - part.res_prefix[item_base]);
@@ -209,88 +210,22 @@ static hy_status enqueue_partition(const hy_db *db, hy_scratch *sc, const Partit
     return fail(HY_OK);
 }
 
-// Per-target scores (and ends) for every sequence, optionally folding the best-hit key. The
-// int32 items of this query run on the scratch's second stream, concurrently with the int16x2
-// pairs, and are joined back before the call's later work.
-// P is the int16x2 pair arithmetic of the database's layout (Pair16: Gathered, PairTab16:
-// Precomputed).
-template <class P>
-static hy_status enqueue_scores_p(const hy_db *db, hy_scratch *sc, const uint8_t *d_query,
-                                  uint64_t qlen, bool ends, unsigned long long *key, int32_t *scores) {
-    hy_status st;
-    const QuerySplit split = split_for_query(db, qlen);
-    const int gpb = BLOCK / MAIN_G;
-    const bool forked = split.n_i32 > 0;
-    if (forked) {
-        HY_CK(cudaEventRecord(sc->ev_fork, sc->stream));
-        HY_CK(cudaStreamWaitEvent(sc->stream2, sc->ev_fork, 0));
-        const int gpb32 = BLOCK / MAIN_G32;
-        const int blocks = (int)((split.n_i32 + gpb32 - 1) / gpb32);
-        st = enqueue_partition<Single32, MAIN_G32, MAIN_R32>(db, sc, db->p32, 0, split.n_i32, d_query,
-                                                          qlen, ends, key, scores, sc->d_prof32,
-                                                          sc->d_bnd32, nullptr, blocks, BLOCK,
-                                                          sc->stream2);
-        if (st != HY_OK) return st;
-        HY_CK(cudaEventRecord(sc->ev_join, sc->stream2));
-    }
-    if (split.k0 < db->p16.n_items) {
-        const int blocks = (int)((db->p16.n_items - split.k0 + gpb - 1) / gpb);
-        // Rows per lane by query length: more rows amortise the per-step work, fewer keep the
-        // padding of a short query's single pass small. An alphabet whose two pass slices do not
-        // fit in shared memory runs with 8 rows, from the profile in global memory if need be.
-        int rows = bulk_rows(qlen, db->mode == MODE_SW && !ends);
-        const size_t slice = profile_slice_row_bytes<P>(db->al) * MAIN_G;
-        if (2 * slice * rows + 16 > db->smem_limit) rows = 8;
-#define HY_BULK(RR)                                                                              \
-    enqueue_partition<P, MAIN_G, RR>(db, sc, db->p16, split.k0, db->p16.n_items, d_query,        \
-                                          qlen, ends, key, scores, sc->d_prof16, sc->d_bnd16,    \
-                                          nullptr, blocks, BLOCK, sc->stream)
-        st = rows == 8 ? HY_BULK(8) : rows == 16 ? HY_BULK(16) : HY_BULK(32);
-#undef HY_BULK
-        if (st != HY_OK) return st;
-    }
-    if (forked) HY_CK(cudaStreamWaitEvent(sc->stream, sc->ev_join, 0));
-    return fail(HY_OK);
-}
-
-static hy_status enqueue_scores(const hy_db *db, hy_scratch *sc, const uint8_t *d_query,
-                                uint64_t qlen, bool ends, unsigned long long *key, int32_t *scores) {
-    return db->layout == HY_LAYOUT_PRECOMPUTED
-               ? enqueue_scores_p<PairTab16>(db, sc, d_query, qlen, ends, key, scores)
-               : enqueue_scores_p<Pair16>(db, sc, d_query, qlen, ends, key, scores);
-}
-
-// The winner's item: its int16x2 pair when that pair ran packed for this query (pair >= k0),
-// else its int32 single (the 2*k0 longest sequences). The other slot gets NO_INDEX. A key of 0
-// means no item recorded a hit (a scan kernel gave up on a bounded wait): no winner then.
-__global__ void winner_loc_kernel(const unsigned long long *key, const uint32_t *rank, uint32_t k0,
-                                  uint32_t *win) {
-    if (*key == 0) {
-        win[0] = win[1] = NO_INDEX;
-        return;
-    }
-    const uint32_t idx = ~(uint32_t)(*key & 0xffffffffu);
-    const uint32_t r = rank[idx];
-    const bool packed = r / 2 >= k0;
-    win[0] = packed ? r / 2 : NO_INDEX;
-    win[1] = packed ? NO_INDEX : r;
-}
-
-// The band kernel on one block, or on a cluster of `blocks` blocks (at most 8, the portable
+// The band kernel on one block an item, or on a cluster of `blocks` blocks (at most 8, the portable
 // cluster size every launch shape of one block per SM can be given).
 template <class A, int R, int MODE, bool GPROF>
-static cudaError_t launch_band_mode(const ScanParams &p, int warps, int blocks, size_t smem, cudaStream_t st) {
+static cudaError_t launch_band_mode(const ScanParams &p, int warps, int blocks, size_t smem, uint32_t items,
+                                    cudaStream_t st) {
     auto kern = band_kernel<A, R, MODE, GPROF>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     if (GPROF || blocks <= 1) {
-        kern<<<1, 32 * warps, smem, st>>>(p);
+        kern<<<items, 32 * warps, smem, st>>>(p);
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.gridDim = dim3(items * (unsigned)blocks);
     cfg.blockDim = dim3(32u * (unsigned)warps);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -352,12 +287,12 @@ static BandShape band_plan(uint64_t qlen, uint64_t al, size_t smem_limit, QueryP
 }
 
 template <class A>
-static cudaError_t launch_band(int mode, const BandShape &sh, const ScanParams &p, cudaStream_t st) {
+static cudaError_t launch_band(int mode, const BandShape &sh, const ScanParams &p, uint32_t items, cudaStream_t st) {
 #define HY_BAND_CASE(M)                                                                                     \
     case M:                                                                                                 \
-        return sh.gprof             ? launch_band_mode<A, WIN_R, M, true>(p, sh.warps, 1, sh.smem, st)      \
-               : sh.rows == WIN_R   ? launch_band_mode<A, WIN_R, M, false>(p, sh.warps, sh.blocks, sh.smem, st) \
-                                    : launch_band_mode<A, BAND_FEW_ROWS, M, false>(p, sh.warps, sh.blocks, sh.smem, st);
+        return sh.gprof             ? launch_band_mode<A, WIN_R, M, true>(p, sh.warps, 1, sh.smem, items, st)      \
+               : sh.rows == WIN_R   ? launch_band_mode<A, WIN_R, M, false>(p, sh.warps, sh.blocks, sh.smem, items, st) \
+                                    : launch_band_mode<A, BAND_FEW_ROWS, M, false>(p, sh.warps, sh.blocks, sh.smem, items, st);
     switch (mode) {
         HY_BAND_CASE(MODE_SW)
         HY_BAND_CASE(MODE_NW)
@@ -370,6 +305,14 @@ static cudaError_t launch_band(int mode, const BandShape &sh, const ScanParams &
 }
 
 }  // namespace hy
+
+namespace hy {
+static void debug_forms(const hy_db *db, uint64_t qlen, bool ends, uint32_t out[5]);
+}
+
+extern "C" void hy_debug_scan_forms(const hy_db *db, uint64_t qlen, int ends, uint32_t out[5]) {
+    hy::debug_forms(db, qlen, ends != 0, out);
+}
 
 extern "C" void hy_debug_band_shape(uint32_t pass_bytes, int32_t n_passes, uint64_t smem_limit, int32_t out[4]) {
     hy::QueryPlan qp;
@@ -384,22 +327,23 @@ extern "C" void hy_debug_band_shape(uint32_t pass_bytes, int32_t n_passes, uint6
 
 namespace hy {
 
-// End positions of the single item *item_ptr with the block-cooperative band kernel.
+// Scores and end positions of the single item *item_ptr, or of the items [item_base, item_end) (a
+// block or cluster each), with the band kernel on stream `st`; optionally folds the best-hit key.
 template <class A>
-static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &part,
-                              uint32_t item_end, const uint8_t *d_query, uint64_t qlen,
-                              uint8_t *prof, void *bnd, const uint32_t *item_ptr) {
+static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &part, uint32_t item_base,
+                              uint32_t item_end, const uint8_t *d_query, uint64_t qlen, unsigned long long *key,
+                              int32_t *scores, uint8_t *prof, void *bnd, const uint32_t *item_ptr, cudaStream_t st) {
     const bool i16 = A::NH == 2;
     QueryPlan qp;
     const BandShape sh = band_plan<A>(qlen, db->al, db->smem_limit, qp);
     const int32_t lim = i16 ? lim16(db) : LIM32;
     if (sh.rows == WIN_R)
-        HY_CK((launch_profile<A, WIN_G, WIN_R>(db, d_query, qlen, qp, lim, prof, sc->stream)));
+        HY_CK((launch_profile<A, WIN_G, WIN_R>(db, d_query, qlen, qp, lim, prof, st)));
     else
-        HY_CK((launch_profile<A, WIN_G, BAND_FEW_ROWS>(db, d_query, qlen, qp, lim, prof, sc->stream)));
+        HY_CK((launch_profile<A, WIN_G, BAND_FEW_ROWS>(db, d_query, qlen, qp, lim, prof, st)));
     ScanParams p{};
     p.meta = part.d_meta;
-    p.item_base = 0;
+    p.item_base = item_base;
     p.n_items = item_end;
     p.item_ptr = item_ptr;
     p.res = part.d_res;
@@ -412,16 +356,165 @@ static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &
     p.ge = db->ge;
     p.sentinel = i16 ? (-32768 + db->ge) : (INT32_MIN / 4);
     p.boundary = bnd;
-    p.scores = sc->d_scores;
+    p.scores = scores;
     p.qend = sc->d_qend;
     p.tend = sc->d_tend;
-    p.best_key = nullptr;
+    p.best_key = key;
     p.err = sc->d_err;
     p.wait_polls = wait_polls();
     set_extents<A>(p, db, part, part.total_cols);
-    HY_CK(launch_band<A>(db->mode, sh, p, sc->stream));
+    HY_CK(launch_band<A>(db->mode, sh, p, item_ptr ? 1 : item_end - item_base, st));
     sc->launches += qp.n_passes > 0 ? 2 : 1;
     return fail(HY_OK);
+}
+
+// Blocks of 256 threads of a launch over the items [base, end) with G lanes each.
+static int blocks_for(uint32_t base, uint32_t end, int G, int threads = BLOCK) {
+    const uint32_t per = (uint32_t)(threads / G);
+    return (int)((end - base + per - 1) / per);
+}
+
+// Threads of a wide block with 16 rows per lane: two slices of a large alphabet leave an SM one block,
+// of 512 threads then.
+template <class P>
+static int wide_threads(const hy_db *db, uint64_t qlen) {
+    const QueryPlan qp = plan_for<P>(qlen, WIDE_MAX_RPP, db->al);
+    return scan_slices(qp.n_passes) * (size_t)qp.pass_bytes > 110 * 1024 ? 512 : BLOCK;
+}
+
+// The pairs [base, end) a warp each (or 16 lanes: queries of at most 64 residues), on `st`.
+template <class P>
+static hy_status enqueue_wide(const hy_db *db, hy_scratch *sc, const ScanForms &f, uint32_t base, uint32_t end,
+                              const uint8_t *d_query, uint64_t qlen, bool ends, unsigned long long *key,
+                              int32_t *scores, cudaStream_t st) {
+#define HY_WIDE(GG, RR, THREADS)                                                                              \
+    enqueue_partition<P, GG, RR>(db, sc, db->p16, base, end, d_query, qlen, ends, key, scores, sc->d_profx16, \
+                                 sc->d_bnd16, nullptr, blocks_for(base, end, GG, THREADS), THREADS, st)
+    if (f.wide_g == 16) return HY_WIDE(16, 4, BLOCK);
+    switch (f.wide_r) {
+    case 4: return HY_WIDE(32, 4, BLOCK);
+    case 8: return HY_WIDE(32, 8, BLOCK);
+    case 12: return HY_WIDE(32, 12, BLOCK);
+    }
+    return wide_threads<P>(db, qlen) > BLOCK ? HY_WIDE(32, 16, 512) : HY_WIDE(32, 16, BLOCK);
+#undef HY_WIDE
+}
+
+// Rows per lane of the bulk kernel: more rows amortise the per-step work, fewer keep the padding of a
+// short query's single pass small. An alphabet whose two pass slices do not fit in shared memory runs
+// with 8 rows, from the profile in global memory if need be.
+template <class P>
+static int bulk_rows_for(const hy_db *db, uint64_t qlen, bool ends) {
+    const int rows = bulk_rows(qlen, db->mode == MODE_SW, ends);
+    return 2 * profile_slice_row_bytes<P>(db->al) * MAIN_G * rows + scan_extra_smem(2, rows, db->mode, ends, BLOCK) >
+                   db->smem_limit
+               ? 8
+               : rows;
+}
+
+// The forms a scan's items run in. An alphabet whose wide slices do not fit in shared memory keeps
+// every pair in the bulk kernel, and one whose band slices do not, every item out of the band kernel.
+template <class P>
+static ScanForms forms_for(const hy_db *db, const QuerySplit &split, uint64_t qlen, bool ends) {
+    int g, r;
+    wide_shape(qlen, db->mode == MODE_SW, &g, &r);
+    if (r == 16 && wide_threads<P>(db, qlen) > BLOCK && db->mode == MODE_SW && ends) r = 8;  // no room for the copies
+    ScanForms f = scan_forms(db, split, qlen, ends, bulk_rows_for<P>(db, qlen, ends), g, r,
+                             r == 16 ? wide_threads<P>(db, qlen) : BLOCK);
+    QueryPlan bp;
+    if (band_plan<P>(qlen, db->al, db->smem_limit, bp).rows != BAND_FEW_ROWS) f.band_end = split.k0;
+    if (band_plan<Single32>(qlen, db->al, db->smem_limit, bp).rows != BAND_FEW_ROWS) f.band32 = false;
+    const QueryPlan wp = plan_for<P>(qlen, g * r, db->al);
+    if (scan_slices(wp.n_passes) * (size_t)wp.pass_bytes + scan_extra_smem(2, r, db->mode, ends, BLOCK) > db->smem_limit)
+        f.wide_end = f.band_end;
+    f.wide_end = std::max(f.wide_end, f.band_end);
+    return f;
+}
+
+// Per-target scores (and ends) for every sequence, optionally folding the best-hit key. The int32
+// items and the band items run on the scratch's second stream and the pairs a warp each on its third,
+// concurrently with the bulk, and are joined back before the call's later work. P is the int16x2 pair
+// arithmetic of the database's layout (Pair16: Gathered, PairTab16: Precomputed).
+template <class P>
+static hy_status enqueue_scores_p(const hy_db *db, hy_scratch *sc, const uint8_t *d_query,
+                                  uint64_t qlen, bool ends, unsigned long long *key, int32_t *scores) {
+    hy_status st;
+    const QuerySplit split = split_for_query(db, qlen);
+    const ScanForms forms = forms_for<P>(db, split, qlen, ends);
+    const bool fork2 = split.n_i32 > 0 || forms.band_end > split.k0, fork3 = forms.wide_end > forms.band_end;
+    if (fork2 || fork3) HY_CK(cudaEventRecord(sc->ev_fork, sc->stream));
+    if (fork2) {
+        HY_CK(cudaStreamWaitEvent(sc->stream2, sc->ev_fork, 0));
+        if (split.n_i32 > 0) {
+            st = forms.band32
+                     ? enqueue_band<Single32>(db, sc, db->p32, 0, split.n_i32, d_query, qlen, key, scores, sc->d_profw32,
+                                              sc->d_bnd32, nullptr, sc->stream2)
+                     : enqueue_partition<Single32, MAIN_G32, MAIN_R32>(
+                           db, sc, db->p32, 0, split.n_i32, d_query, qlen, ends, key, scores, sc->d_prof32, sc->d_bnd32,
+                           nullptr, blocks_for(0, split.n_i32, MAIN_G32), BLOCK, sc->stream2);
+            if (st != HY_OK) return st;
+        }
+        if (forms.band_end > split.k0) {
+            st = enqueue_band<P>(db, sc, db->p16, split.k0, forms.band_end, d_query, qlen, key, scores, sc->d_profw16,
+                                 sc->d_bnd16, nullptr, sc->stream2);
+            if (st != HY_OK) return st;
+        }
+        HY_CK(cudaEventRecord(sc->ev_join, sc->stream2));
+    }
+    if (fork3) {
+        HY_CK(cudaStreamWaitEvent(sc->stream3, sc->ev_fork, 0));
+        st = enqueue_wide<P>(db, sc, forms, forms.band_end, forms.wide_end, d_query, qlen, ends, key, scores, sc->stream3);
+        if (st != HY_OK) return st;
+        HY_CK(cudaEventRecord(sc->ev_join3, sc->stream3));
+    }
+    if (forms.wide_end < db->p16.n_items) {
+        const int rows = bulk_rows_for<P>(db, qlen, ends);
+#define HY_BULK(RR)                                                                                         \
+    enqueue_partition<P, MAIN_G, RR>(db, sc, db->p16, forms.wide_end, db->p16.n_items, d_query, qlen, ends, \
+                                     key, scores, sc->d_prof16, sc->d_bnd16, nullptr,                       \
+                                     blocks_for(forms.wide_end, db->p16.n_items, MAIN_G), BLOCK, sc->stream)
+        st = rows == 8 ? HY_BULK(8) : rows == 16 ? HY_BULK(16) : HY_BULK(32);
+#undef HY_BULK
+        if (st != HY_OK) return st;
+    }
+    if (fork2) HY_CK(cudaStreamWaitEvent(sc->stream, sc->ev_join, 0));
+    if (fork3) HY_CK(cudaStreamWaitEvent(sc->stream, sc->ev_join3, 0));
+    return fail(HY_OK);
+}
+
+static void debug_forms(const hy_db *db, uint64_t qlen, bool ends, uint32_t out[5]) {
+    const QuerySplit split = split_for_query(db, qlen);
+    const ScanForms f = db->layout == HY_LAYOUT_PRECOMPUTED ? forms_for<PairTab16>(db, split, qlen, ends)
+                                                            : forms_for<Pair16>(db, split, qlen, ends);
+    out[0] = split.n_i32;
+    out[1] = f.band32 ? 1 : 0;
+    out[2] = f.band_end - split.k0;
+    out[3] = f.wide_end - f.band_end;
+    out[4] = db->p16.n_items - f.wide_end;
+}
+
+static hy_status enqueue_scores(const hy_db *db, hy_scratch *sc, const uint8_t *d_query,
+                                uint64_t qlen, bool ends, unsigned long long *key, int32_t *scores) {
+    return db->layout == HY_LAYOUT_PRECOMPUTED
+               ? enqueue_scores_p<PairTab16>(db, sc, d_query, qlen, ends, key, scores)
+               : enqueue_scores_p<Pair16>(db, sc, d_query, qlen, ends, key, scores);
+}
+
+// The winner's item: its int16x2 pair when that pair ran packed for this query (pair >= k0),
+// else its int32 single (the 2*k0 longest sequences). The other slot gets NO_INDEX, and both where the
+// band kernel ran the item and has left its ends: pairs below band_end, with band32 the int32 items. A
+// key of 0 means no item recorded a hit (a scan kernel gave up on a bounded wait): no winner then.
+__global__ void winner_loc_kernel(const unsigned long long *key, const uint32_t *rank, uint32_t k0,
+                                  uint32_t band_end, bool band32, uint32_t *win) {
+    if (*key == 0) {
+        win[0] = win[1] = NO_INDEX;
+        return;
+    }
+    const uint32_t idx = ~(uint32_t)(*key & 0xffffffffu);
+    const uint32_t r = rank[idx];
+    const bool packed = r / 2 >= k0;
+    win[0] = packed && r / 2 >= band_end ? r / 2 : NO_INDEX;
+    win[1] = packed || band32 ? NO_INDEX : r;
 }
 
 // Device buffers of the long-pair band paths, grow-only, per calling thread and device.
@@ -563,7 +656,7 @@ static hy_status band_pair_enqueue(BandPairContext &c, const uint8_t *d_q, uint6
     p.n_seqs = slot + 1;
     p.letters = (uint32_t)Single32::letters((int64_t)al);
     HY_CK(cudaEventRecord(c.ev[0], st));
-    HY_CK(launch_band<Single32>(mode, sh, p, st));
+    HY_CK(launch_band<Single32>(mode, sh, p, 1, st));
     HY_CK(cudaEventRecord(c.ev[1], st));
     return fail(HY_OK);
 }
@@ -655,20 +748,21 @@ static hy_status enqueue_scan(const hy_db *db, hy_scratch *sc, const uint8_t *d_
         // End positions of the winner only (src/database.rs:186-197): rerun its item with
         // position tracking on a whole block (the band kernel).
         const QuerySplit split = split_for_query(db, qlen);
-        winner_loc_kernel<<<1, 1, 0, sc->stream>>>(sc->d_key, db->d_rank, split.k0, sc->d_win);
+        const bool tab = db->layout == HY_LAYOUT_PRECOMPUTED;
+        const ScanForms forms = tab ? forms_for<PairTab16>(db, split, qlen, false) : forms_for<Pair16>(db, split, qlen, false);
+        winner_loc_kernel<<<1, 1, 0, sc->stream>>>(sc->d_key, db->d_rank, split.k0, forms.band_end, forms.band32, sc->d_win);
         HY_CK(cudaGetLastError());
         ++sc->launches;
-        if (split.k0 < db->p16.n_items) {
-            st = db->layout == HY_LAYOUT_PRECOMPUTED
-                     ? enqueue_band<PairTab16>(db, sc, db->p16, db->p16.n_items, d_query, qlen,
-                                               sc->d_profw16, sc->d_bnd16, sc->d_win)
-                     : enqueue_band<Pair16>(db, sc, db->p16, db->p16.n_items, d_query, qlen,
-                                            sc->d_profw16, sc->d_bnd16, sc->d_win);
+        if (forms.band_end < db->p16.n_items) {
+            st = tab ? enqueue_band<PairTab16>(db, sc, db->p16, 0, db->p16.n_items, d_query, qlen, nullptr, sc->d_scores,
+                                               sc->d_profw16, sc->d_bnd16, sc->d_win, sc->stream)
+                     : enqueue_band<Pair16>(db, sc, db->p16, 0, db->p16.n_items, d_query, qlen, nullptr, sc->d_scores,
+                                            sc->d_profw16, sc->d_bnd16, sc->d_win, sc->stream);
             if (st != HY_OK) return st;
         }
-        if (split.n_i32 > 0) {
-            st = enqueue_band<Single32>(db, sc, db->p32, split.n_i32, d_query, qlen, sc->d_profw32,
-                                        sc->d_bnd32, sc->d_win + 1);
+        if (split.n_i32 > 0 && !forms.band32) {
+            st = enqueue_band<Single32>(db, sc, db->p32, 0, split.n_i32, d_query, qlen, nullptr, sc->d_scores,
+                                        sc->d_profw32, sc->d_bnd32, sc->d_win + 1, sc->stream);
             if (st != HY_OK) return st;
         }
     }
@@ -1075,7 +1169,7 @@ uint64_t hy_db_scratch_bytes(const hy_db *db) {
     const uint64_t mq = std::max<uint64_t>(db->mql, 1);
     uint64_t b = mq + 3 * 4 * db->n_seqs + 64 + sizeof(hy_hit);
     const uint64_t pr = pair_slice_row_bytes(db), sr = profile_slice_row_bytes<Single32>(db->al);
-    b += npass(mq, BULK_MAX_RPP) * BULK_MAX_RPP * pr;
+    b += npass(mq, BULK_MAX_RPP) * BULK_MAX_RPP * pr + npass(mq, WIDE_MAX_RPP) * WIDE_MAX_RPP * pr;
     b += npass(mq, MAIN_G32 * MAIN_R32) * MAIN_G32 * MAIN_R32 * sr;
     b += npass(mq, WIN_G * WIN_R) * WIN_G * WIN_R * (pr + sr);
     if (mq > (uint64_t)std::min({MAIN_G * 8, MAIN_G * MAIN_R16, MAIN_G32 * MAIN_R32, WIN_G * WIN_R}))
@@ -1102,23 +1196,28 @@ hy_status hy_scratch_create(const hy_db *db, hy_scratch **out) {
     int prio_low = 0, prio_high = 0;
     ck(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
     ck(cudaStreamCreateWithPriority(&sc->stream2, cudaStreamNonBlocking, prio_high));
+    ck(cudaStreamCreateWithPriority(&sc->stream3, cudaStreamNonBlocking, prio_high));
     ck(cudaEventCreateWithFlags(&sc->ev_fork, cudaEventDisableTiming));
     ck(cudaEventCreateWithFlags(&sc->ev_join, cudaEventDisableTiming));
+    ck(cudaEventCreateWithFlags(&sc->ev_join3, cudaEventDisableTiming));
     ck(hy::dev_malloc(&sc->d_query, mq));
     auto prof_bytes = [&](int rpp, size_t slice_row_bytes) {
         return std::max<uint64_t>(1, npass(mq, rpp) * rpp * slice_row_bytes);
     };
     const uint64_t pr = pair_slice_row_bytes(db), sr = profile_slice_row_bytes<Single32>(db->al);
     ck(hy::dev_malloc(&sc->d_prof16, prof_bytes(BULK_MAX_RPP, pr)));
+    ck(hy::dev_malloc(&sc->d_profx16, prof_bytes(WIDE_MAX_RPP, pr)));
     ck(hy::dev_malloc(&sc->d_prof32, prof_bytes(MAIN_G32 * MAIN_R32, sr)));
     ck(hy::dev_malloc(&sc->d_profw16, prof_bytes(WIN_G * WIN_R, pr)));
     ck(hy::dev_malloc(&sc->d_profw32, prof_bytes(WIN_G * WIN_R, sr)));
     const bool multipass = mq > (uint64_t)std::min({MAIN_G * 8, MAIN_G * MAIN_R16, MAIN_G32 * MAIN_R32, WIN_G * WIN_R});
     ck(hy::dev_malloc(&sc->d_bnd16, multipass ? std::max<uint64_t>(8, 8 * db->p16.total_cols) : 8));
     ck(hy::dev_malloc(&sc->d_bnd32, multipass ? std::max<uint64_t>(8, 8 * db->p32.total_cols) : 8));
-    ck(hy::dev_malloc(&sc->d_scores, 4 * n));
-    ck(hy::dev_malloc(&sc->d_qend, 4 * n));
-    ck(hy::dev_malloc(&sc->d_tend, 4 * n));
+    ck(hy::dev_malloc(&sc->d_scores, 3 * 4 * n));  // then the ends: one copy back for all three
+    if (sc->d_scores) {
+        sc->d_qend = sc->d_scores + n;
+        sc->d_tend = sc->d_qend + n;
+    }
     ck(hy::dev_malloc(&sc->d_key, 64));
     ck(hy::dev_malloc(&sc->d_win, 64));
     ck(hy::dev_malloc(&sc->d_hit, sizeof(hy_hit)));
@@ -1148,14 +1247,13 @@ void hy_scratch_destroy(hy_scratch *sc) {
     tb_context_destroy(sc->tb);
     hy::dev_free(sc->d_query);
     hy::dev_free(sc->d_prof16);
+    hy::dev_free(sc->d_profx16);
     hy::dev_free(sc->d_prof32);
     hy::dev_free(sc->d_profw16);
     hy::dev_free(sc->d_profw32);
     hy::dev_free(sc->d_bnd16);
     hy::dev_free(sc->d_bnd32);
     hy::dev_free(sc->d_scores);
-    hy::dev_free(sc->d_qend);
-    hy::dev_free(sc->d_tend);
     hy::dev_free(sc->d_key);
     hy::dev_free(sc->d_win);
     hy::dev_free(sc->d_hit);
@@ -1173,7 +1271,10 @@ void hy_scratch_destroy(hy_scratch *sc) {
     if (sc->stream2) cudaStreamSynchronize(sc->stream2);
     if (sc->ev_fork) cudaEventDestroy(sc->ev_fork);
     if (sc->ev_join) cudaEventDestroy(sc->ev_join);
+    if (sc->ev_join3) cudaEventDestroy(sc->ev_join3);
     if (sc->stream2) cudaStreamDestroy(sc->stream2);
+    if (sc->stream3) cudaStreamSynchronize(sc->stream3);
+    if (sc->stream3) cudaStreamDestroy(sc->stream3);
     if (sc->stream) cudaStreamDestroy(sc->stream);
     delete sc;
 }
@@ -1307,11 +1408,7 @@ hy_status hy_scan_all(const hy_db *db, hy_scratch *sc, const uint8_t *query, uin
         hy_status s2;
         if ((s2 = issue_query(sc, qlen)) != HY_OK) return s2;
         if ((s2 = enqueue_scores(db, sc, sc->d_query, qlen, ends, nullptr, sc->d_scores)) != HY_OK) return s2;
-        HY_CK(cudaMemcpyAsync(sc->h_out, sc->d_scores, 4 * n, cudaMemcpyDeviceToHost, sc->stream));
-        if (ends) {
-            HY_CK(cudaMemcpyAsync(sc->h_out + n, sc->d_qend, 4 * n, cudaMemcpyDeviceToHost, sc->stream));
-            HY_CK(cudaMemcpyAsync(sc->h_out + 2 * n, sc->d_tend, 4 * n, cudaMemcpyDeviceToHost, sc->stream));
-        }
+        HY_CK(cudaMemcpyAsync(sc->h_out, sc->d_scores, (ends ? 3 : 1) * 4 * n, cudaMemcpyDeviceToHost, sc->stream));
         return issue_err_back(sc);
     });
     if (st != HY_OK) return st;

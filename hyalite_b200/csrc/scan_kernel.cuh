@@ -765,7 +765,60 @@ struct Sweep2 {
     typename A::V Gp[R], E[R];        // G of the previous column and E, per row slot
     typename A::V diag;               // G of the row above the lane at the column before j0
     typename A::V botG[2], botF[2];   // this lane's last row at columns j0, j1, for lane L + 1
+    // End tracking: a value that this lane's cells must exceed to be the answer, and per half the first
+    // of the two columns that last did (-1: none this pass).
+    typename A::V pbest;
+    int32_t pcol[2];
 };
+
+// End tracking costs a comparison a step. A cell can be the answer only if it exceeds every earlier
+// column of its lane, and is no worse than the cells of the lanes above up to the step's columns (equal:
+// it may win by its column) and of the passes before. Where a step has such a cell in some half, both
+// columns' rows are copied to shared memory (`copy`: the lane's uint4s `stride` apart, R / 2 a half), and
+// the cell is looked up in the copy at the pass's end. (scan_all of 50,000 protein sequences, a query of
+// 900: 26.1 ms with a predicate and two selects a cell on 8 lanes a pair, 6.4 with the length forms and a
+// comparison a column, 5.6 so.)
+template <class A, int R>
+__device__ __forceinline__ void sweep2_track(Sweep2<A, R> &sw, const typename A::V (&g0)[R], const typename A::V (&g1)[R],
+                                             const typename A::V cm, const int32_t j, uint4 *copy, const int stride) {
+    if (cm == sw.pbest) return;
+#pragma unroll
+    for (int h = 0; h < A::NH; ++h) {
+        const uint32_t mask = A::NH == 1 ? 0xffffffffu : h ? 0xffff0000u : 0xffffu;
+        if (((uint32_t)cm ^ (uint32_t)sw.pbest) & mask) {
+#pragma unroll
+            for (int c = 0; c < R / 4; ++c) {
+                copy[(h * (R / 2) + c) * stride] = make_uint4((uint32_t)g0[4 * c], (uint32_t)g0[4 * c + 1],
+                                                              (uint32_t)g0[4 * c + 2], (uint32_t)g0[4 * c + 3]);
+                copy[(h * (R / 2) + R / 4 + c) * stride] = make_uint4((uint32_t)g1[4 * c], (uint32_t)g1[4 * c + 1],
+                                                                      (uint32_t)g1[4 * c + 2], (uint32_t)g1[4 * c + 3]);
+            }
+            sw.pcol[h] = j;
+        }
+    }
+    sw.pbest = cm;
+}
+
+// The lane's tracked cells of a pass whose first row of this lane is row0, as candidates: the first
+// column's rows, then the second's, so the first cell with the copy's maximum.
+template <class A, int R>
+__device__ __forceinline__ void sweep2_tracked(const Sweep2<A, R> &sw, const int32_t row0, const int32_t go,
+                                               const uint4 *copy, const int stride, Cand (&cand)[2]) {
+#pragma unroll
+    for (int h = 0; h < A::NH; ++h) {
+        if (sw.pcol[h] < 0) continue;
+        int32_t best = INT32_MIN;
+        int at = 0;
+        for (int c = 0; c < R / 2; ++c) {
+            const uint4 v = copy[(h * (R / 2) + c) * stride];
+            const int32_t g[4] = {A::get(v.x, h), A::get(v.y, h), A::get(v.z, h), A::get(v.w, h)};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (g[e] > best) best = g[e], at = 4 * c + e;
+        }
+        consider(cand[h], best + go, sw.pcol[h] + at / R, row0 + at % R);
+    }
+}
 
 // One column of R rows: E, F, H, G in place; returns the last row's G and F.
 template <class A, int G, int R>
@@ -801,14 +854,16 @@ __device__ __forceinline__ void sweep2_column(Sweep2<A, R> &sw, const int a, con
 
 // Both columns of a step, interleaved one row apart (row r of column j0 with row r - 1 of column
 // j1, which needs rows r - 1 of column j0 only): the same values as sweep2_column twice, with the
-// two columns' dependency chains side by side in the instruction stream.
-template <class A, int G, int R>
+// two columns' dependency chains side by side in the instruction stream. With ENDS column j0's G is kept
+// in g0.
+template <class A, int G, int R, bool ENDS>
 __device__ __forceinline__ void sweep2_both(Sweep2<A, R> &sw, const int a0, const int b0, const int a1,
                                             const int b1, const int lane, const uint8_t *prof_a,
                                             const uint8_t *prof_b, const typename A::V upG0,
                                             const typename A::V upF0, const typename A::V upG1,
                                             const typename A::V upF1, const typename A::V negge,
-                                            const typename A::V neggo, typename A::V &best) {
+                                            const typename A::V neggo, typename A::V &best,
+                                            typename A::V (&g0)[R]) {
     typedef typename A::V V;
     V p0a[A::EPV], p0b[A::EPV], p1a[A::EPV], p1b[A::EPV];
     V g_up0 = upG0, f0 = upF0, gd0 = sw.diag, hprev0 = A::splat(0);
@@ -825,6 +880,7 @@ __device__ __forceinline__ void sweep2_both(Sweep2<A, R> &sw, const int a0, cons
             const V g = A::vadd(h, neggo);
             gd0 = sw.Gp[r];
             sw.Gp[r] = g;
+            if (ENDS) g0[r] = g;
             g_up0 = g;
             if (r & 1)
                 best = A::vmax3(best, hprev0, g);
@@ -858,12 +914,12 @@ __device__ __forceinline__ void sweep2_both(Sweep2<A, R> &sw, const int a0, cons
 // Step s of one lane (see above). The residue codes of columns j0, j1 come as one 32-bit word
 // (`codes`) and, for lane 0 after the first pass, the boundary values of both columns as one
 // 16-byte word (`up`: G, F of j0, then of j1). CHECKED steps test each column against [1, w].
-template <class A, int G, int R, bool CHECKED>
+template <class A, int G, int R, bool CHECKED, bool ENDS>
 __device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const int s, const int lane, const int32_t w,
                                             const uint8_t *prof_a, const uint8_t *prof_b,
                                             const bool first_pass, const bool last_pass,
                                             typename A::V *bnd, const SweepConst<A> &k,
-                                            typename A::V &best, const uint32_t codes, const uint4 up) {
+                                            typename A::V &best, const uint32_t codes, const uint4 up, uint4 *copy) {
     typedef typename A::V V;
     constexpr int CODE_BITS = TwoCodes<A>::BITS;
     constexpr uint32_t CODE_MASK = (1u << CODE_BITS) - 1u;
@@ -886,24 +942,37 @@ __device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const int s, const
         }
     }
     int a, b;
+    if (ENDS) {
+        const V upB = __shfl_up_sync(0xffffffffu, sw.pbest, 1, G);
+        if (lane > 0) sw.pbest = A::vmax(sw.pbest, A::vadd(upB, A::splat(-1)));
+        best = sw.pbest;
+    }
+    V g0[R];
     if (!CHECKED) {
         // Both columns live: interleaved (measured 0.6% faster than one after the other).
         int a1, b1;
         A::residues((typename A::RES)(codes & CODE_MASK), a, b);
         A::residues((typename A::RES)(codes >> CODE_BITS), a1, b1);
-        sweep2_both<A, G, R>(sw, a, b, a1, b1, lane, prof_a, prof_b, upG0, upF0, upG1, upF1, k.negge, k.neggo,
-                             best);
+        sweep2_both<A, G, R, ENDS>(sw, a, b, a1, b1, lane, prof_a, prof_b, upG0, upF0, upG1, upF1, k.negge, k.neggo,
+                                   best, g0);
+        if (ENDS) sweep2_track<A, R>(sw, g0, sw.Gp, best, j0, copy, (int)blockDim.x);
     } else {
         if (live0) {
             A::residues((typename A::RES)(codes & CODE_MASK), a, b);
             sweep2_column<A, G, R>(sw, a, b, lane, prof_a, prof_b, upG0, upF0, sw.diag, k.negge, k.neggo, best,
                                    sw.botG[0], sw.botF[0]);
+            if (ENDS) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) g0[r] = sw.Gp[r];
+            }
         }
         if (live1) {
             A::residues((typename A::RES)(codes >> CODE_BITS), a, b);
             sweep2_column<A, G, R>(sw, a, b, lane, prof_a, prof_b, upG1, upF1, upG0, k.negge, k.neggo, best,
                                    sw.botG[1], sw.botF[1]);
         }
+        // (A dead second column leaves the first one's rows in Gp.)
+        if (ENDS && live0) sweep2_track<A, R>(sw, g0, sw.Gp, best, j0, copy, (int)blockDim.x);
     }
     if (live0) sw.diag = live1 ? upG1 : upG0;
     if (lane == G - 1 && !last_pass && live0)
@@ -929,11 +998,12 @@ __device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const int s, const
 //
 // Every thread of the block calls it with the block's `phase` (see scan_unit). Returns false if a
 // profile copy did not arrive in time (the error flag is then set and the block must stop).
-template <class A, int G, int R>
+template <class A, int G, int R, bool ENDS>
 __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane, const int W, const int wfast,
                                             const int32_t w, const typename A::RES *__restrict__ res,
                                             typename A::V *bnd, uint8_t *smem, uint64_t *bars,
-                                            uint32_t &phase, const typename A::V Sv, typename A::V &best) {
+                                            uint32_t &phase, const typename A::V Sv, typename A::V &best,
+                                            Cand (&cand)[2]) {
     typedef typename A::V V;
     typedef typename TwoCodes<A>::W W2;
     const int n_passes = p.n_passes;
@@ -952,6 +1022,16 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
             sw.E[r] = Sv;
         }
         sw.diag = k.top_free_g;
+        sw.pcol[0] = sw.pcol[1] = -1;
+        // In a later pass a cell as good as the passes before may still win, by its column.
+        if (ENDS) sw.pbest = A::vmax(k.neggo, A::vadd(sw.pbest, A::splat(-1)));
+    };
+    sw.pbest = k.neggo;  // H = 0: only a cell above the border's 0 is tracked
+    uint4 *copy = reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(bars) + 16) + threadIdx.x;
+    // This lane is done with pass `pass`.
+    auto tracked = [&](int pass) {
+        if constexpr (ENDS)
+            sweep2_tracked<A, R>(sw, p.vrow0 + pass * (G * R) + lane * R, p.go, copy, (int)blockDim.x, cand);
     };
     reset();
     sw.botG[0] = sw.botG[1] = sw.botF[0] = sw.botF[1] = A::splat(0);
@@ -967,8 +1047,8 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
     auto checked = [&](int lp, int c) {
         const uint8_t *pa = smem + (size_t)(lp & 1) * p.pass_bytes;
         if (lp < 0) c = -1;
-        sweep2_step<A, G, R, true>(sw, c + lane, lane, w, pa, pa + hi_off, lp == 0, lp == n_passes - 1, bnd, k,
-                                   best, codes_at(c), up_at(c, lp == 0));
+        sweep2_step<A, G, R, true, ENDS>(sw, c + lane, lane, w, pa, pa + hi_off, lp == 0, lp == n_passes - 1, bnd, k,
+                                         best, codes_at(c), up_at(c, lp == 0), copy);
     };
     for (int pass = 0; pass < n_passes; ++pass) {
         const int buf = pass & 1;
@@ -978,10 +1058,10 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
             __syncwarp();
             for (int t = 0; t < G - 1; ++t) {
                 const bool fresh = lane <= t;  // this lane has entered pass `pass`
-                if (fresh && lane == t && pass > 0) reset();
+                if (fresh && lane == t && pass > 0) tracked(pass - 1), reset();
                 checked(fresh ? pass : pass - 1, fresh ? t - lane : W + t - lane);
             }
-            if (lane == G - 1 && pass > 0) reset();  // lane G-1 enters at the first interior step
+            if (lane == G - 1 && pass > 0) tracked(pass - 1), reset();  // lane G-1 enters at the first interior step
         }
         if (__syncthreads_or(!ok)) {
             // This pass's copy and, in the first pass, the second one are still outstanding.
@@ -1007,20 +1087,21 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
             for (; s + 1 < fast_hi; s += 2) {
                 c_b = res2[s + 1 - lane];
                 if (up_lane) u_b = bnd4[s + 1];
-                sweep2_step<A, G, R, false>(sw, s, lane, w, pa, pb, first, last, bnd, k, best, c_a, u_a);
+                sweep2_step<A, G, R, false, ENDS>(sw, s, lane, w, pa, pb, first, last, bnd, k, best, c_a, u_a, copy);
                 const int s2 = min(s + 2, fast_hi - 1);
                 c_a = res2[s2 - lane];
                 if (up_lane) u_a = bnd4[s2];
-                sweep2_step<A, G, R, false>(sw, s + 1, lane, w, pa, pb, first, last, bnd, k, best, c_b, u_b);
+                sweep2_step<A, G, R, false, ENDS>(sw, s + 1, lane, w, pa, pb, first, last, bnd, k, best, c_b, u_b, copy);
             }
             if (s < fast_hi)
-                sweep2_step<A, G, R, false>(sw, s, lane, w, pa, pb, first, last, bnd, k, best, c_a, u_a);
+                sweep2_step<A, G, R, false, ENDS>(sw, s, lane, w, pa, pb, first, last, bnd, k, best, c_a, u_a, copy);
         }
         for (int s = fast_hi; s < W; ++s) checked(pass, s - lane);
     }
     // The last pass's drain: lanes L > t finish their columns W + t - L.
     if (W > 0)
         for (int t = 0; t < G - 1; ++t) checked(lane > t ? n_passes - 1 : -1, W + t - lane);
+    if (n_passes > 0) tracked(n_passes - 1);
     __syncthreads();  // both profile buffers are free for the block's next unit
     return true;
 }
@@ -1084,14 +1165,19 @@ __device__ __forceinline__ void finish_item(const int lane, const bool active, c
     }
 }
 
-// Whether a scan launch shape runs the two-column sweep: SW scores of int16x2 pairs or int32 items
-// with at most 16 rows per lane. Measured on the protein benchmark: for the pairs as fast as one
+// Rows per lane the two-column sweep takes: up to 16; with ends from 12 on (with fewer rows the
+// comparison a step outweighs what the second column saves: 64-residue queries against 5,000 reads 77 us
+// a call with one column a step, 90 with two).
+__host__ __device__ constexpr bool scan_two_col_rows(int rows, bool ends) { return rows <= 16 && (!ends || rows >= 12); }
+
+// Whether a scan launch shape runs the two-column sweep: SW of int16x2 pairs or int32 items with at
+// most 16 rows per lane. Measured on the protein benchmark: for the pairs as fast as one
 // column of 32 rows, with half the per-lane state and 10% faster on 64-residue DNA queries; for the
 // int32 items of a 5000-residue query 1014 against 594 GCUPS (two independent column chains per
 // lane for their latency-bound warps).
 template <class A, int R, int MODE, bool ENDS, bool GPROF>
 __host__ __device__ constexpr bool two_col_form() {
-    return TwoCodes<A>::OK && ModeFlags<MODE>::local && !ENDS && !GPROF && R <= 16;
+    return TwoCodes<A>::OK && ModeFlags<MODE>::local && !GPROF && scan_two_col_rows(R, ENDS);
 }
 
 #ifdef HY_BOUNDS
@@ -1186,10 +1272,11 @@ __device__ __forceinline__ bool scan_unit(const ScanParams &p, const uint32_t it
         if (p.n_passes > 1) bulk_load(smem + p.pass_bytes, p.profile + p.pass_bytes, p.pass_bytes, &bars[1]);
     }
     if constexpr (two_col_form<A, R, MODE, ENDS, GPROF>()) {
-        // Column pairs a pass: at least 2G (the boundary row's read-after-write distance).
-        const int W = wmax == 0 ? 0 : max((int)(wmax + 1) / 2, 2 * G);
-        if (!sweep2_item<A, G, R>(p, lane, W, min(W, w_min / 2), (int32_t)meta.w, res, bnd, smem, bars, phase, Sv,
-                                  best))
+        // Column pairs a pass: at least 2G (the boundary row's read-after-write distance), and with one
+        // pass the G - 1 of the fill.
+        const int W = wmax == 0 ? 0 : max((int)(wmax + 1) / 2, p.n_passes > 1 ? 2 * G : G - 1);
+        if (!sweep2_item<A, G, R, ENDS>(p, lane, W, min(W, w_min / 2), (int32_t)meta.w, res, bnd, smem, bars, phase,
+                                        Sv, best, cand))
             return false;
     } else {
         for (int pass = 0; pass < p.n_passes; ++pass) {
@@ -1224,19 +1311,40 @@ __device__ __forceinline__ bool scan_unit(const ScanParams &p, const uint32_t it
     return true;
 }
 
+// Threads a block of a launch shape may have: 512 for the pairs a warp each with 16 rows per lane,
+// whose two slices of a large alphabet leave an SM one block.
+template <class A, int G, int R>
+constexpr int scan_max_threads() {
+    return A::NH == 2 && G == 32 && R == 16 ? 512 : 256;
+}
+
 // Resident 256-thread blocks per SM each launch shape is compiled for (its register budget).
 // The two-column sweep of 16 rows per lane is compiled for two blocks (measured faster than three
 // with the spills three would need).
 template <class A, int G, int R, bool TWO_COL = false>
 constexpr int scan_min_blocks() {
-    return A::NH == 1 ? 2 : (G == 8 && R == 8) ? 4 : (G == 8 && R == 32) ? 2 : (TWO_COL && R == 16) ? 2 : 3;
+    return A::NH == 1                                       ? 2
+           : (G == 8 && R == 8) || R == 4                   ? 4
+           : (G == 8 && R == 32) || (TWO_COL && R == 16 && G == 8) ? 2
+           : scan_max_threads<A, G, R>() == 512             ? 1
+           : R == 12                                        ? 2
+                                                            : 3;
 }
 
+// Shared memory of a scan block besides its pass slices: the mbarriers and, where the two-column sweep
+// tracks ends, each lane's copied columns.
+inline size_t scan_extra_smem(int halves, int rows, int mode, bool ends, int threads) {
+    return 16 + (mode == MODE_SW && ends && scan_two_col_rows(rows, ends) ? (size_t)halves * 2 * rows * 4 * threads : 0);
+}
+
+// Pass slices a launch keeps in shared memory.
+__host__ __device__ inline uint32_t scan_slices(int32_t n_passes) { return n_passes > 1 ? 2 : 1; }
+
 template <class A, int G, int R, int MODE, bool ENDS, bool GPROF = false>
-__global__ void __launch_bounds__(256, (scan_min_blocks<A, G, R, two_col_form<A, R, MODE, ENDS, GPROF>()>()))
+__global__ void __launch_bounds__((scan_max_threads<A, G, R>()), (scan_min_blocks<A, G, R, two_col_form<A, R, MODE, ENDS, GPROF>()>()))
     scan_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (GPROF ? 0 : 2 * (size_t)p.pass_bytes));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (GPROF ? 0 : scan_slices(p.n_passes) * (size_t)p.pass_bytes));
     const int gpb = blockDim.x / G;
     uint32_t first, end;
     if (p.item_ptr) {
@@ -1802,6 +1910,7 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                 p.scores[idx] = c.s;
                 p.qend[idx] = c.row - 1;
                 p.tend[idx] = c.col - 1;
+                if (p.best_key) atomicMax(p.best_key, hit_key(c.s, idx));
             }
         }
     }
@@ -1818,8 +1927,9 @@ constexpr int band_max_warps() {
 template <class A, int R, int MODE, bool GPROF = false>
 __global__ void __launch_bounds__(32 * band_max_warps<R>(), 1) band_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const uint32_t item = *p.item_ptr;
-    if (item == NO_INDEX || item >= p.n_items) return;  // the same for every thread of the block
+    // The item *item_ptr, or an item a cluster.
+    const uint32_t item = p.item_ptr ? *p.item_ptr : p.item_base + blockIdx.x / (uint32_t)cluster_size();
+    if (item == NO_INDEX || item >= p.n_items) return;  // the same for every thread of the cluster
     const int W = blockDim.x / 32;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + band_smem_bytes(W, GPROF ? 0 : p.pass_bytes, R)) - BAND_BARS;
     if (threadIdx.x == 0) {
