@@ -65,9 +65,9 @@ __device__ __forceinline__ void class_range(const BatchQuery &bq, int cls, uint3
 
 // One persistent kernel per launch class: blocks take units off the class queue until it is empty.
 // Shared memory: the two profile mbarriers, then two pass slices of the largest pass of the batch.
-// SW_ONLY: the SW classes, compiled for the SW sweep alone (the two-column form's register budget).
+// SW_ONLY: the SW classes, compiled for the SW sweep alone.
 template <class A, int G, int R, int PK, bool SW_ONLY = false>
-__global__ void __launch_bounds__(256, (scan_min_blocks<A, G, R, SW_ONLY && two_col_form<A, R, MODE_SW, false, false>()>()))
+__global__ void __launch_bounds__(256, (scan_min_blocks<A, G, R, two_col_form<A, R, MODE_SW, false, false>()>()))
     batch_scan_kernel(const ClassLaunch L) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t s_unit;
@@ -259,7 +259,7 @@ static void plan_kinds(const hy_db *db, uint64_t qlen, bool ends, const BatchCon
     // SW scores (the bulk classes never record ends) take the plain scan's two-column shapes; the
     // other modes the tuned thresholds.
     if (db->mode == MODE_SW)
-        k.rows = bulk_rows(qlen, true);
+        k.rows = bulk_rows(qlen);
     else
         k.rows = (int64_t)qlen <= cfg.rows8_max ? 8 : (int64_t)qlen <= cfg.rows16_max ? 16 : 32;
     const QuerySplit &sp = k.split;
@@ -569,7 +569,7 @@ static hy_status time_config(hy_batch *b, const BatchItem *items, uint32_t n, co
 // Coordinate search: the rows-per-lane thresholds first (at the default split), then the split.
 static hy_status tune(hy_batch *b, const BatchItem *items, uint32_t n, uint32_t stride,
                       BatchConfig *best_cfg, double *best_ms) {
-    static const int32_t rows_c[][2] = {{64, 192}, {0, 256}, {128, 512}, {0, 0}, {64, 64}, {32, 128}};
+    static const int32_t rows_c[][2] = {{64, BATCH_ROWS16_ALL}, {0, BATCH_ROWS16_ALL}, {128, BATCH_ROWS16_ALL}, {64, 1024}, {64, 192}};
     static const uint32_t long_c[] = {1024, 2048, 4096};
     BatchConfig best = b->cfg;
     float best_t = 1e30f;

@@ -40,9 +40,10 @@ struct BatchCtl {
     uint32_t chunk_stride;    // 1, or k to run only every k-th chunk (autotuner samples)
 };
 
+constexpr int32_t BATCH_ROWS16_ALL = 1 << 30;  // beyond every query length
 struct BatchConfig {
-    int32_t rows8_max = 64;    // queries up to this length: 8 rows per lane
-    int32_t rows16_max = 192;  // up to this length: 16 rows per lane; longer: 32
+    int32_t rows8_max = 64;                  // queries up to this length: 8 rows per lane, two columns a step
+    int32_t rows16_max = BATCH_ROWS16_ALL;   // up to this length: 16 rows, two columns; longer: 32 rows, one
     uint32_t long_w = LONG_W;  // pairs wider than this run one warp each
 };
 

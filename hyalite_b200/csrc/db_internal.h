@@ -30,20 +30,17 @@ constexpr int LONG_R = 8;
 constexpr uint32_t LONG_W = 4096;
 constexpr uint32_t NO_LONG_SPLIT = 0xffffffffu;
 constexpr int BLOCK = 256;
-// Rows per lane of the bulk int16x2 kernel for a query of length qlen (passes of MAIN_G * rows).
-// SW runs the two-column sweep at 8 or 16 rows per lane: 16 unless 8 pads the query to so
-// many fewer rows that it wins at 8 rows' rate per padded row (measured 0.853 of 16 rows' rate,
-// 4813 against 5641 GCUPS for 1000-residue queries on the protein benchmark: 150 residues take 192
-// rows at 8 against 256 at 16). The other kinds run one column of up to 32 rows.
-inline int bulk_rows(uint64_t qlen, bool two_col, bool ends = false) {
+// Rows per lane of the bulk int16x2 kernel for a query of length qlen (passes of MAIN_G * rows): the
+// two-column sweep at 8 or 16 rows per lane, 16 unless 8 pads the query to so many fewer rows that it
+// wins at 8 rows' rate per padded row (measured 0.853 of 16 rows' rate, 4813 against 5641 GCUPS for
+// 1000-residue queries on the protein benchmark: 150 residues take 192 rows at 8 against 256 at 16).
+inline int bulk_rows(uint64_t qlen, bool local_ends = false) {
     if (qlen <= 64) return 8;
-    if (two_col && ends) return 16;  // the two-column sweep tracks ends from 12 rows per lane on
-    if (two_col) {
-        const uint64_t rows8 = (qlen + 63) / 64 * 64, rows16 = (qlen + 127) / 128 * 128;
-        return 7 * rows8 < 6 * rows16 ? 8 : 16;
-    }
-    return qlen <= 192 ? 16 : 32;
+    if (local_ends) return 16;  // the two-column sweep tracks ends from 12 rows per lane on
+    const uint64_t rows8 = (qlen + 63) / 64 * 64, rows16 = (qlen + 127) / 128 * 128;
+    return 7 * rows8 < 6 * rows16 ? 8 : 16;
 }
+// Rows of a pass slice that LayoutChoice::Auto sizes the pair table for.
 constexpr int BULK_MAX_RPP = 8 * 32;
 constexpr int WIDE_MAX_RPP = 32 * 16;
 constexpr size_t BAND_SMEM_BUDGET = 200 * 1024;
@@ -204,11 +201,11 @@ struct ScanForms {
 
 // Lanes and rows per lane of the wide form: one pass of the fewest rows up to 512 rows, longer queries
 // in passes of 512 or 256 rows by padded rows at their rates (8 rows 0.853 of 16 rows').
-inline void wide_shape(uint64_t qlen, bool two_col, int *g, int *r) {
+inline void wide_shape(uint64_t qlen, int *g, int *r) {
     *g = qlen <= 64 ? 16 : 32;
     if (qlen <= 128) *r = 4;
     else if (qlen <= 256) *r = 8;
-    else if (qlen <= 384 && two_col) *r = 12;
+    else if (qlen <= 384) *r = 12;
     else if (qlen <= 512) *r = 16;
     else *r = 7 * ((qlen + 255) / 256 * 256) < 6 * ((qlen + 511) / 512 * 512) ? 8 : 16;
 }
@@ -223,8 +220,8 @@ struct ScanCost {
     // Instructions of one item's chain: passes of g * r rows over w columns.
     double chain(uint64_t qlen, int g, int r, double w) const {
         const double passes = (double)((qlen + (uint64_t)(g * r) - 1) / (uint64_t)(g * r));
-        if (mode == MODE_SW && scan_two_col_rows(r, ends)) return (passes * w / 2 + g) * ((ends ? 110.0 : 50.0) + 15.1 * r);
-        return passes * (w + g) * (50.0 + (mode == MODE_SW ? 13.0 : 9.0) * r);
+        if (!scan_two_col_rows(r, mode, ends)) return passes * (w + g) * (50.0 + 13.0 * r);
+        return (passes * w / 2 + g) * (mode != MODE_SW ? 55.0 + 14.1 * r : (ends ? 110.0 : 50.0) + 15.1 * r);
     }
 };
 constexpr double COST_SCHEDULERS = 148 * 4, COST_BUSY = 1.46, COST_ALONE = 2.2, COST_FORM = 16000;

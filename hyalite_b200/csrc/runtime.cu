@@ -405,7 +405,7 @@ static hy_status enqueue_wide(const hy_db *db, hy_scratch *sc, const ScanForms &
 // with 8 rows, from the profile in global memory if need be.
 template <class P>
 static int bulk_rows_for(const hy_db *db, uint64_t qlen, bool ends) {
-    const int rows = bulk_rows(qlen, db->mode == MODE_SW, ends);
+    const int rows = bulk_rows(qlen, db->mode == MODE_SW && ends);
     return 2 * profile_slice_row_bytes<P>(db->al) * MAIN_G * rows + scan_extra_smem(2, rows, db->mode, ends, BLOCK) >
                    db->smem_limit
                ? 8
@@ -417,7 +417,7 @@ static int bulk_rows_for(const hy_db *db, uint64_t qlen, bool ends) {
 template <class P>
 static ScanForms forms_for(const hy_db *db, const QuerySplit &split, uint64_t qlen, bool ends) {
     int g, r;
-    wide_shape(qlen, db->mode == MODE_SW, &g, &r);
+    wide_shape(qlen, &g, &r);
     if (r == 16 && wide_threads<P>(db, qlen) > BLOCK && db->mode == MODE_SW && ends) r = 8;  // no room for the copies
     ScanForms f = scan_forms(db, split, qlen, ends, bulk_rows_for<P>(db, qlen, ends), g, r,
                              r == 16 ? wide_threads<P>(db, qlen) : BLOCK);
@@ -473,7 +473,7 @@ static hy_status enqueue_scores_p(const hy_db *db, hy_scratch *sc, const uint8_t
     enqueue_partition<P, MAIN_G, RR>(db, sc, db->p16, forms.wide_end, db->p16.n_items, d_query, qlen, ends, \
                                      key, scores, sc->d_prof16, sc->d_bnd16, nullptr,                       \
                                      blocks_for(forms.wide_end, db->p16.n_items, MAIN_G), BLOCK, sc->stream)
-        st = rows == 8 ? HY_BULK(8) : rows == 16 ? HY_BULK(16) : HY_BULK(32);
+        st = rows == 8 ? HY_BULK(8) : HY_BULK(16);
 #undef HY_BULK
         if (st != HY_OK) return st;
     }

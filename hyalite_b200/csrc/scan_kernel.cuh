@@ -117,6 +117,8 @@ struct Pair16 {
         uint32_t h = (uint16_t)(int16_t)x;
         return h | (h << 16);
     }
+    // splat of a value that fits.
+    __device__ __forceinline__ static V pack(int32_t x) { return __byte_perm((uint32_t)x, 0, 0x1010); }
     __device__ __forceinline__ static V addmax(V a, V b, V c) { return __viaddmax_s16x2(a, b, c); }
     __device__ __forceinline__ static V vmax(V a, V b) { return __vmaxs2(a, b); }
     __device__ __forceinline__ static V vmax3(V a, V b, V c) { return __vimax3_s16x2(a, b, c); }
@@ -233,6 +235,7 @@ struct Single32 {
     __device__ __forceinline__ static V splat(int64_t x) {
         return (V)(x < VMIN ? VMIN : (x > VMAX ? VMAX : x));
     }
+    __device__ __forceinline__ static V pack(int32_t x) { return x; }
     __device__ __forceinline__ static V addmax(V a, V b, V c) { return __viaddmax_s32(a, b, c); }
     __device__ __forceinline__ static V vmax(V a, V b) { return max(a, b); }
     __device__ __forceinline__ static V vmax3(V a, V b, V c) { return __vimax3_s32(a, b, c); }
@@ -743,13 +746,15 @@ __device__ __forceinline__ void sweep_pass(const int lane, const int steps, cons
     sweep_end<A, R, MODE, ENDS>(sw, row0, go, cand);
 }
 
-// ---- two columns per step: the SW score sweep of int16x2 pairs and int32 items ------------------
+// ---- two columns per step: the sweep of int16x2 pairs and int32 items ---------------------------
 //
 // Lane L works on columns j0 = 2(s - L) + 1 and j1 = j0 + 1 at step s, R rows each: the per-step
 // work (shuffles, residue and boundary loads, loop control) is spread over 2R rows of work while a
 // lane keeps only R rows of state, and the F chains of the two columns (column j1 one row behind
 // column j0) give the scheduler two independent dependency chains. Long form of the recurrence
-// (E, F, H = max(d, E, F, 0), G = H - go); the running maximum is kept on G.
+// (E, F, H = max(d, E, F), in local mode also max with 0, G = H - go); the running maximum is kept on
+// G. The modes that answer in the last row track it once a step; those that answer in a sequence's last
+// column do so in checked steps, which every step is that may hold one.
 
 // The residue codes of two adjacent columns as one load: two 16-bit pair codes (int16x2 pairs) or
 // two 8-bit residues (int32 items). OK: the lane arithmetic has a two-column form.
@@ -769,9 +774,10 @@ struct Sweep2 {
     // of the two columns that last did (-1: none this pass).
     typename A::V pbest;
     int32_t pcol[2];
+    typename A::V lastG;  // the last query row's running maximum (lane G - 1, last pass)
 };
 
-// End tracking costs a comparison a step. A cell can be the answer only if it exceeds every earlier
+// End tracking (local mode) costs a comparison a step. A cell can be the answer only if it exceeds every earlier
 // column of its lane, and is no worse than the cells of the lanes above up to the step's columns (equal:
 // it may win by its column) and of the passes before. Where a step has such a cell in some half, both
 // columns' rows are copied to shared memory (`copy`: the lane's uint4s `stride` apart, R / 2 a half), and
@@ -821,7 +827,7 @@ __device__ __forceinline__ void sweep2_tracked(const Sweep2<A, R> &sw, const int
 }
 
 // One column of R rows: E, F, H, G in place; returns the last row's G and F.
-template <class A, int G, int R>
+template <class A, int G, int R, bool LOCAL>
 __device__ __forceinline__ void sweep2_column(Sweep2<A, R> &sw, const int a, const int b, const int lane,
                                               const uint8_t *prof_a, const uint8_t *prof_b,
                                               typename A::V g_up, typename A::V f, typename A::V gd,
@@ -837,26 +843,28 @@ __device__ __forceinline__ void sweep2_column(Sweep2<A, R> &sw, const int a, con
         sw.E[r] = A::addmax(sw.E[r], negge, sw.Gp[r]);
         f = A::addmax(f, negge, g_up);
         const V d = A::diag(gd, pa[r % A::EPV], pb[r % A::EPV]);
-        const V h = A::vmax3_relu(d, sw.E[r], f);
+        const V h = LOCAL ? A::vmax3_relu(d, sw.E[r], f) : A::vmax3(d, sw.E[r], f);
         const V g = A::vadd(h, neggo);
         gd = sw.Gp[r];
         sw.Gp[r] = g;
         g_up = g;
-        if (r & 1)
-            best = A::vmax3(best, hprev, g);
-        else
-            hprev = g;
+        if (LOCAL) {
+            if (r & 1)
+                best = A::vmax3(best, hprev, g);
+            else
+                hprev = g;
+        }
     }
-    if (R & 1) best = A::vmax(best, hprev);
+    if (LOCAL && (R & 1)) best = A::vmax(best, hprev);
     outG = g_up;
     outF = f;
 }
 
 // Both columns of a step, interleaved one row apart (row r of column j0 with row r - 1 of column
 // j1, which needs rows r - 1 of column j0 only): the same values as sweep2_column twice, with the
-// two columns' dependency chains side by side in the instruction stream. With ENDS column j0's G is kept
+// two columns' dependency chains side by side in the instruction stream. With TRACK column j0's G is kept
 // in g0.
-template <class A, int G, int R, bool ENDS>
+template <class A, int G, int R, bool LOCAL, bool TRACK>
 __device__ __forceinline__ void sweep2_both(Sweep2<A, R> &sw, const int a0, const int b0, const int a1,
                                             const int b1, const int lane, const uint8_t *prof_a,
                                             const uint8_t *prof_b, const typename A::V upG0,
@@ -876,16 +884,18 @@ __device__ __forceinline__ void sweep2_both(Sweep2<A, R> &sw, const int a0, cons
             sw.E[r] = A::addmax(sw.E[r], negge, sw.Gp[r]);
             f0 = A::addmax(f0, negge, g_up0);
             const V d = A::diag(gd0, p0a[r % A::EPV], p0b[r % A::EPV]);
-            const V h = A::vmax3_relu(d, sw.E[r], f0);
+            const V h = LOCAL ? A::vmax3_relu(d, sw.E[r], f0) : A::vmax3(d, sw.E[r], f0);
             const V g = A::vadd(h, neggo);
             gd0 = sw.Gp[r];
             sw.Gp[r] = g;
-            if (ENDS) g0[r] = g;
+            if (TRACK) g0[r] = g;
             g_up0 = g;
-            if (r & 1)
-                best = A::vmax3(best, hprev0, g);
-            else
-                hprev0 = g;
+            if (LOCAL) {
+                if (r & 1)
+                    best = A::vmax3(best, hprev0, g);
+                else
+                    hprev0 = g;
+            }
         }
         if (t >= 1) {  // column j1, row t - 1
             const int r = t - 1;
@@ -893,34 +903,39 @@ __device__ __forceinline__ void sweep2_both(Sweep2<A, R> &sw, const int a0, cons
             sw.E[r] = A::addmax(sw.E[r], negge, sw.Gp[r]);
             f1 = A::addmax(f1, negge, g_up1);
             const V d = A::diag(gd1, p1a[r % A::EPV], p1b[r % A::EPV]);
-            const V h = A::vmax3_relu(d, sw.E[r], f1);
+            const V h = LOCAL ? A::vmax3_relu(d, sw.E[r], f1) : A::vmax3(d, sw.E[r], f1);
             const V g = A::vadd(h, neggo);
             gd1 = sw.Gp[r];
             sw.Gp[r] = g;
             g_up1 = g;
-            if (r & 1)
-                best = A::vmax3(best, hprev1, g);
-            else
-                hprev1 = g;
+            if (LOCAL) {
+                if (r & 1)
+                    best = A::vmax3(best, hprev1, g);
+                else
+                    hprev1 = g;
+            }
         }
     }
-    if (R & 1) best = A::vmax3(best, hprev0, hprev1);
+    if (LOCAL && (R & 1)) best = A::vmax3(best, hprev0, hprev1);
     sw.botG[0] = g_up0;
     sw.botF[0] = f0;
     sw.botG[1] = g_up1;
     sw.botF[1] = f1;
 }
 
-// Step s of one lane (see above). The residue codes of columns j0, j1 come as one 32-bit word
-// (`codes`) and, for lane 0 after the first pass, the boundary values of both columns as one
-// 16-byte word (`up`: G, F of j0, then of j1). CHECKED steps test each column against [1, w].
-template <class A, int G, int R, bool CHECKED, bool ENDS>
-__device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const int s, const int lane, const int32_t w,
-                                            const uint8_t *prof_a, const uint8_t *prof_b,
-                                            const bool first_pass, const bool last_pass,
-                                            typename A::V *bnd, const SweepConst<A> &k,
-                                            typename A::V &best, const uint32_t codes, const uint4 up, uint4 *copy) {
+// Step s of one lane (see above), whose first row is row0. The residue codes of columns j0, j1 come as
+// one 32-bit word (`codes`) and, for lane 0 after the first pass, the boundary values of both columns
+// as one 16-byte word (`up`: G, F of j0, then of j1). CHECKED steps test each column against [1, w].
+template <class A, int G, int R, int MODE, bool CHECKED, bool ENDS>
+__device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const ScanParams &p, const int s, const int lane,
+                                            const int32_t w, const uint32_t (&n)[2], const uint8_t *prof_a,
+                                            const uint8_t *prof_b, const int32_t row0, const bool first_pass,
+                                            const bool last_pass, typename A::V *bnd, const SweepConst<A> &k,
+                                            typename A::V &best, Cand (&cand)[2], const uint32_t codes, const uint4 up,
+                                            uint4 *copy) {
     typedef typename A::V V;
+    typedef ModeFlags<MODE> Fl;
+    constexpr bool TRACK = Fl::local && ENDS;
     constexpr int CODE_BITS = TwoCodes<A>::BITS;
     constexpr uint32_t CODE_MASK = (1u << CODE_BITS) - 1u;
     const int32_t j0 = 2 * (s - lane) + 1;
@@ -932,7 +947,13 @@ __device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const int s, const
     const bool live1 = !CHECKED || (j0 + 1 >= 1 && j0 + 1 <= w);
     if (lane == 0) {
         if (first_pass) {
-            upG0 = upG1 = k.top_free_g;
+            if (Fl::top_free) {
+                upG0 = upG1 = k.top_free_g;
+            } else {
+                // G of H(0, j) = -go - (j - 1) ge (columns past the item may wrap: never used).
+                upG0 = A::pack(-2 * p.go - (j0 - 1) * p.ge);
+                upG1 = A::vadd(upG0, k.negge);
+            }
             upF0 = upF1 = k.Sv;
         } else {
             upG0 = up.x;
@@ -942,37 +963,72 @@ __device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const int s, const
         }
     }
     int a, b;
-    if (ENDS) {
+    if (TRACK) {
         const V upB = __shfl_up_sync(0xffffffffu, sw.pbest, 1, G);
         if (lane > 0) sw.pbest = A::vmax(sw.pbest, A::vadd(upB, A::splat(-1)));
         best = sw.pbest;
     }
+    const bool last_lane = last_pass && lane == G - 1;
     V g0[R];
     if (!CHECKED) {
         // Both columns live: interleaved (measured 0.6% faster than one after the other).
         int a1, b1;
         A::residues((typename A::RES)(codes & CODE_MASK), a, b);
         A::residues((typename A::RES)(codes >> CODE_BITS), a1, b1);
-        sweep2_both<A, G, R, ENDS>(sw, a, b, a1, b1, lane, prof_a, prof_b, upG0, upF0, upG1, upF1, k.negge, k.neggo,
-                                   best, g0);
-        if (ENDS) sweep2_track<A, R>(sw, g0, sw.Gp, best, j0, copy, (int)blockDim.x);
+        sweep2_both<A, G, R, Fl::local, TRACK>(sw, a, b, a1, b1, lane, prof_a, prof_b, upG0, upF0, upG1, upF1, k.negge,
+                                               k.neggo, best, g0);
+        if (TRACK) sweep2_track<A, R>(sw, g0, sw.Gp, best, j0, copy, (int)blockDim.x);
+        if (Fl::last_row && last_lane) {
+            const V m = A::vmax3(sw.lastG, sw.botG[0], sw.botG[1]);
+            if (m != sw.lastG) {
+#pragma unroll
+                for (int h = 0; h < A::NH; ++h) {
+                    if (j0 <= (int32_t)n[h]) consider(cand[h], A::get(sw.botG[0], h) + p.go, j0, p.qlen);
+                    if (j0 + 1 <= (int32_t)n[h]) consider(cand[h], A::get(sw.botG[1], h) + p.go, j0 + 1, p.qlen);
+                }
+                sw.lastG = m;
+            }
+        }
     } else {
+        // Candidates of column j, whose rows are in Gp and last row's G is g.
+        auto answers = [&](const int32_t j, const V g) {
+            if ((Fl::last_row || Fl::corner) && last_lane) {
+                sw.lastG = A::vmax(sw.lastG, g);
+#pragma unroll
+                for (int h = 0; h < A::NH; ++h) {
+                    const int32_t nh = (int32_t)n[h];
+                    if (Fl::last_row ? (j <= nh) : (j == nh)) consider(cand[h], A::get(g, h) + p.go, j, p.qlen);
+                }
+            }
+            if (Fl::last_col) {
+#pragma unroll
+                for (int h = 0; h < A::NH; ++h) {
+                    if (j == (int32_t)n[h]) {
+#pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            if (row0 + r >= 1) consider(cand[h], A::get(sw.Gp[r], h) + p.go, j, row0 + r);
+                    }
+                }
+            }
+        };
         if (live0) {
             A::residues((typename A::RES)(codes & CODE_MASK), a, b);
-            sweep2_column<A, G, R>(sw, a, b, lane, prof_a, prof_b, upG0, upF0, sw.diag, k.negge, k.neggo, best,
-                                   sw.botG[0], sw.botF[0]);
-            if (ENDS) {
+            sweep2_column<A, G, R, Fl::local>(sw, a, b, lane, prof_a, prof_b, upG0, upF0, sw.diag, k.negge, k.neggo,
+                                              best, sw.botG[0], sw.botF[0]);
+            answers(j0, sw.botG[0]);
+            if (TRACK) {
 #pragma unroll
                 for (int r = 0; r < R; ++r) g0[r] = sw.Gp[r];
             }
         }
         if (live1) {
             A::residues((typename A::RES)(codes >> CODE_BITS), a, b);
-            sweep2_column<A, G, R>(sw, a, b, lane, prof_a, prof_b, upG1, upF1, upG0, k.negge, k.neggo, best,
-                                   sw.botG[1], sw.botF[1]);
+            sweep2_column<A, G, R, Fl::local>(sw, a, b, lane, prof_a, prof_b, upG1, upF1, upG0, k.negge, k.neggo, best,
+                                              sw.botG[1], sw.botF[1]);
+            answers(j0 + 1, sw.botG[1]);
         }
         // (A dead second column leaves the first one's rows in Gp.)
-        if (ENDS && live0) sweep2_track<A, R>(sw, g0, sw.Gp, best, j0, copy, (int)blockDim.x);
+        if (TRACK && live0) sweep2_track<A, R>(sw, g0, sw.Gp, best, j0, copy, (int)blockDim.x);
     }
     if (live0) sw.diag = live1 ? upG1 : upG0;
     if (lane == G - 1 && !last_pass && live0)
@@ -998,13 +1054,16 @@ __device__ __forceinline__ void sweep2_step(Sweep2<A, R> &sw, const int s, const
 //
 // Every thread of the block calls it with the block's `phase` (see scan_unit). Returns false if a
 // profile copy did not arrive in time (the error flag is then set and the block must stop).
-template <class A, int G, int R, bool ENDS>
+template <class A, int G, int R, int MODE, bool ENDS>
 __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane, const int W, const int wfast,
-                                            const int32_t w, const typename A::RES *__restrict__ res,
+                                            const int32_t w, const uint32_t (&n)[2],
+                                            const typename A::RES *__restrict__ res,
                                             typename A::V *bnd, uint8_t *smem, uint64_t *bars,
                                             uint32_t &phase, const typename A::V Sv, typename A::V &best,
                                             Cand (&cand)[2]) {
     typedef typename A::V V;
+    typedef ModeFlags<MODE> Fl;
+    constexpr bool TRACK = Fl::local && ENDS;
     typedef typename TwoCodes<A>::W W2;
     const int n_passes = p.n_passes;
     const uint32_t hi_off = (A::TABLES - 1) * (p.pass_bytes / A::TABLES);
@@ -1014,26 +1073,31 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
     k.Sv = Sv;
     k.top_free_g = A::splat(-(int64_t)p.go);
     Sweep2<A, R> sw;
-    // A lane's state at the start of a pass: local mode, the left border is free (H = 0).
-    auto reset = [&]() {
+    auto row0_of = [&](int pass) { return p.vrow0 + pass * (G * R) + lane * R; };
+    // A lane's state at the start of a pass: the left border.
+    auto reset = [&](int pass) {
+        const int32_t row0 = row0_of(pass);
+        auto left = [&](int32_t row) {
+            return Fl::left_free ? k.top_free_g : A::splat((row <= 0 ? 0 : -gap_pen(p.go, p.ge, row)) - p.go);
+        };
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            sw.Gp[r] = k.top_free_g;
+            sw.Gp[r] = left(row0 + r);
             sw.E[r] = Sv;
         }
-        sw.diag = k.top_free_g;
+        sw.diag = left(row0 - 1);
         sw.pcol[0] = sw.pcol[1] = -1;
         // In a later pass a cell as good as the passes before may still win, by its column.
-        if (ENDS) sw.pbest = A::vmax(k.neggo, A::vadd(sw.pbest, A::splat(-1)));
+        if (TRACK) sw.pbest = A::vmax(k.neggo, A::vadd(sw.pbest, A::splat(-1)));
     };
     sw.pbest = k.neggo;  // H = 0: only a cell above the border's 0 is tracked
+    sw.lastG = A::splat(A::VMIN);
     uint4 *copy = reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(bars) + 16) + threadIdx.x;
     // This lane is done with pass `pass`.
     auto tracked = [&](int pass) {
-        if constexpr (ENDS)
-            sweep2_tracked<A, R>(sw, p.vrow0 + pass * (G * R) + lane * R, p.go, copy, (int)blockDim.x, cand);
+        if constexpr (TRACK) sweep2_tracked<A, R>(sw, row0_of(pass), p.go, copy, (int)blockDim.x, cand);
     };
-    reset();
+    reset(0);
     sw.botG[0] = sw.botG[1] = sw.botF[0] = sw.botF[1] = A::splat(0);
     const W2 *res2 = reinterpret_cast<const W2 *>(res);  // codes of columns (2i+1, 2i+2)
     const uint4 *bnd4 = reinterpret_cast<const uint4 *>(bnd);          // boundary of the same pair
@@ -1047,8 +1111,8 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
     auto checked = [&](int lp, int c) {
         const uint8_t *pa = smem + (size_t)(lp & 1) * p.pass_bytes;
         if (lp < 0) c = -1;
-        sweep2_step<A, G, R, true, ENDS>(sw, c + lane, lane, w, pa, pa + hi_off, lp == 0, lp == n_passes - 1, bnd, k,
-                                         best, codes_at(c), up_at(c, lp == 0), copy);
+        sweep2_step<A, G, R, MODE, true, ENDS>(sw, p, c + lane, lane, w, n, pa, pa + hi_off, row0_of(lp), lp == 0,
+                                               lp == n_passes - 1, bnd, k, best, cand, codes_at(c), up_at(c, lp == 0), copy);
     };
     for (int pass = 0; pass < n_passes; ++pass) {
         const int buf = pass & 1;
@@ -1058,10 +1122,10 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
             __syncwarp();
             for (int t = 0; t < G - 1; ++t) {
                 const bool fresh = lane <= t;  // this lane has entered pass `pass`
-                if (fresh && lane == t && pass > 0) tracked(pass - 1), reset();
+                if (fresh && lane == t && pass > 0) tracked(pass - 1), reset(pass);
                 checked(fresh ? pass : pass - 1, fresh ? t - lane : W + t - lane);
             }
-            if (lane == G - 1 && pass > 0) tracked(pass - 1), reset();  // lane G-1 enters at the first interior step
+            if (lane == G - 1 && pass > 0) tracked(pass - 1), reset(pass);  // lane G-1 enters at the first interior step
         }
         if (__syncthreads_or(!ok)) {
             // This pass's copy and, in the first pass, the second one are still outstanding.
@@ -1075,6 +1139,7 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
         if (W == 0) continue;
         const uint8_t *pa = smem + (size_t)buf * p.pass_bytes, *pb = pa + hi_off;
         const bool first = pass == 0, last = pass == n_passes - 1;
+        const int32_t row0 = row0_of(pass);
         const int fast_hi = max(G - 1, wfast);
         if (G - 1 < fast_hi) {
             // Two steps an iteration with two sets of registers for the one-step-ahead loads (only
@@ -1087,14 +1152,17 @@ __device__ __forceinline__ bool sweep2_item(const ScanParams &p, const int lane,
             for (; s + 1 < fast_hi; s += 2) {
                 c_b = res2[s + 1 - lane];
                 if (up_lane) u_b = bnd4[s + 1];
-                sweep2_step<A, G, R, false, ENDS>(sw, s, lane, w, pa, pb, first, last, bnd, k, best, c_a, u_a, copy);
+                sweep2_step<A, G, R, MODE, false, ENDS>(sw, p, s, lane, w, n, pa, pb, row0, first, last, bnd, k, best, cand,
+                                                        c_a, u_a, copy);
                 const int s2 = min(s + 2, fast_hi - 1);
                 c_a = res2[s2 - lane];
                 if (up_lane) u_a = bnd4[s2];
-                sweep2_step<A, G, R, false, ENDS>(sw, s + 1, lane, w, pa, pb, first, last, bnd, k, best, c_b, u_b, copy);
+                sweep2_step<A, G, R, MODE, false, ENDS>(sw, p, s + 1, lane, w, n, pa, pb, row0, first, last, bnd, k, best, cand,
+                                                        c_b, u_b, copy);
             }
             if (s < fast_hi)
-                sweep2_step<A, G, R, false, ENDS>(sw, s, lane, w, pa, pb, first, last, bnd, k, best, c_a, u_a, copy);
+                sweep2_step<A, G, R, MODE, false, ENDS>(sw, p, s, lane, w, n, pa, pb, row0, first, last, bnd, k, best, cand,
+                                                        c_a, u_a, copy);
         }
         for (int s = fast_hi; s < W; ++s) checked(pass, s - lane);
     }
@@ -1165,19 +1233,20 @@ __device__ __forceinline__ void finish_item(const int lane, const bool active, c
     }
 }
 
-// Rows per lane the two-column sweep takes: up to 16; with ends from 12 on (with fewer rows the
-// comparison a step outweighs what the second column saves: 64-residue queries against 5,000 reads 77 us
-// a call with one column a step, 90 with two).
-__host__ __device__ constexpr bool scan_two_col_rows(int rows, bool ends) { return rows <= 16 && (!ends || rows >= 12); }
+// Rows per lane the two-column sweep takes: up to 16; tracking ends in local mode from 12 on (with
+// fewer rows the comparison a step outweighs what the second column saves: 64-residue queries against
+// 5,000 reads 77 us a call with one column a step, 90 with two).
+__host__ __device__ constexpr bool scan_two_col_rows(int rows, int mode, bool ends) {
+    return rows <= 16 && (mode != MODE_SW || !ends || rows >= 12);
+}
 
-// Whether a scan launch shape runs the two-column sweep: SW of int16x2 pairs or int32 items with at
-// most 16 rows per lane. Measured on the protein benchmark: for the pairs as fast as one
-// column of 32 rows, with half the per-lane state and 10% faster on 64-residue DNA queries; for the
-// int32 items of a 5000-residue query 1014 against 594 GCUPS (two independent column chains per
-// lane for their latency-bound warps).
+// Whether a scan launch shape runs the two-column sweep. Measured on the protein benchmark (SW scores):
+// for the pairs as fast as one column of 32 rows, with half the per-lane state and 10% faster on
+// 64-residue DNA queries; for the int32 items of a 5000-residue query 1014 against 594 GCUPS (two
+// independent column chains per lane for their latency-bound warps).
 template <class A, int R, int MODE, bool ENDS, bool GPROF>
 __host__ __device__ constexpr bool two_col_form() {
-    return TwoCodes<A>::OK && ModeFlags<MODE>::local && !GPROF && scan_two_col_rows(R, ENDS);
+    return TwoCodes<A>::OK && !GPROF && scan_two_col_rows(R, MODE, ENDS);
 }
 
 #ifdef HY_BOUNDS
@@ -1275,8 +1344,14 @@ __device__ __forceinline__ bool scan_unit(const ScanParams &p, const uint32_t it
         // Column pairs a pass: at least 2G (the boundary row's read-after-write distance), and with one
         // pass the G - 1 of the fill.
         const int W = wmax == 0 ? 0 : max((int)(wmax + 1) / 2, p.n_passes > 1 ? 2 * G : G - 1);
-        if (!sweep2_item<A, G, R, ENDS>(p, lane, W, min(W, w_min / 2), (int32_t)meta.w, res, bnd, smem, bars, phase,
-                                        Sv, best, cand))
+        // Steps before this column pair hold no sequence's last column where the mode answers there.
+        int wfast = min(W, w_min / 2);
+        if constexpr (ModeFlags<MODE>::last_col || ModeFlags<MODE>::corner) {
+            const uint32_t n_low = meta.idx[1] == NO_INDEX ? meta.n[0] : min(meta.n[0], meta.n[1]);
+            wfast = min(wfast, max((int)__reduce_min_sync(0xffffffffu, n_low) - 1, 0) / 2);
+        }
+        if (!sweep2_item<A, G, R, MODE, ENDS>(p, lane, W, wfast, (int32_t)meta.w, meta.n, res, bnd, smem, bars, phase,
+                                              Sv, best, cand))
             return false;
     } else {
         for (int pass = 0; pass < p.n_passes; ++pass) {
@@ -1334,7 +1409,7 @@ constexpr int scan_min_blocks() {
 // Shared memory of a scan block besides its pass slices: the mbarriers and, where the two-column sweep
 // tracks ends, each lane's copied columns.
 inline size_t scan_extra_smem(int halves, int rows, int mode, bool ends, int threads) {
-    return 16 + (mode == MODE_SW && ends && scan_two_col_rows(rows, ends) ? (size_t)halves * 2 * rows * 4 * threads : 0);
+    return 16 + (mode == MODE_SW && ends && scan_two_col_rows(rows, mode, ends) ? (size_t)halves * 2 * rows * 4 * threads : 0);
 }
 
 // Pass slices a launch keeps in shared memory.
