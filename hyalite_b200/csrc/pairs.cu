@@ -39,10 +39,11 @@ constexpr size_t PAIR_SMEM_LIMIT = 200 * 1024;
 // Largest global scratch for group profiles that do not fit in shared memory, per launch.
 constexpr size_t PAIR_GPROF_BYTES = 256ull << 20;
 // Chunks of input pairs the pipeline runs in: up to PAIR_MAX_CHUNKS of at least PAIR_CHUNK_MIN
-// pairs each, and more when that would put over PAIR_CHUNK_BYTES of residues in one chunk (the
+// pairs each (of 65,536 and more, 100,000 mate-rescue pairs were one chunk whose copies and kernels ran
+// one after the other, 12.6 ms a call; in 6 chunks 7.6), and more when that would put over PAIR_CHUNK_BYTES of residues in one chunk (the
 // pinned staging holds three chunks).
 constexpr uint64_t PAIR_MAX_CHUNKS = 16;
-constexpr uint64_t PAIR_CHUNK_MIN = 1 << 16;
+constexpr uint64_t PAIR_CHUNK_MIN = 1 << 14;
 constexpr uint64_t PAIR_CHUNK_BYTES = 512ull << 20;
 // The chunk boundaries of pairs [0, L): cut at equal shares of the residues (query plus target
 // bytes), so that no chunk holds much more than PAIR_CHUNK_BYTES whatever the order of long and
