@@ -27,7 +27,7 @@
 // lane's rows stay within one cache line for many steps (the L2 merges the lanes' 8-byte stores
 // into full sectors before they reach DRAM).
 // The fill also reduces the end cell (Best::consider, src/align.rs:281-327) over the mode's answer
-// region. Walk kernel: one thread per pair follows the codes from the end cell, writing the
+// region. Walk kernel: one warp per pair follows the codes from the end cell, writing the
 // operations backwards into a slot of m + n bytes; a scan and a gather compact the slots.
 #include <string.h>
 
@@ -588,17 +588,24 @@ __device__ inline void tb_end_cell(const TbPair &pr, const TbEnd *ends, int32_t 
     }
 }
 
+// One warp per pair walks from the end cell a run at a time. A walk is a chain of dependent code
+// loads: one thread's loop paid a load's latency every operation. Here the 32 lanes load the next 32
+// cells down the diagonal (or along the gap) at once, a ballot gives how many of them the walk takes,
+// and each lane writes its own operation, so the latency is paid once a run. In local mode lane k's
+// cell value is the current one less the substitution scores of the lanes before it (a warp scan),
+// and the run ends at the first that is 0. (2000 x 2000, 15% mutated: align 1.86 to 1.38 ms a call.)
 template <int MODE>
 __global__ void __launch_bounds__(64) tb_walk_kernel(TbParams P) {
     using F = ModeFlags<MODE>;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
     if (t >= P.n_pairs) return;
     const TbPair pr = P.pairs[t];
     const uint32_t m = pr.m, n = pr.n;
     int32_t bs;
     uint32_t brow, bcol;
     tb_end_cell<MODE>(pr, P.ends, P.go, P.ge, bs, brow, bcol);
-    // Walk. State 0 H, 1 E, 2 F.
+    // Walk, every variable but the lanes' own loads warp-uniform. State 0 H, 1 E, 2 F.
     const uint8_t *D = P.dir + pr.dir_off;
     const uint32_t R = pr.rows, r_log2 = 31 - __clz(R);
     const uint64_t pass_stride = (uint64_t)(n + 31) * 32 * (R / 2);
@@ -607,66 +614,92 @@ __global__ void __launch_bounds__(64) tb_walk_kernel(TbParams P) {
     uint8_t *slot = P.ops + pr.ops_off;
     const uint64_t cap = (uint64_t)m + n;
     uint64_t cnt = 0;
+    // `len` operations `op`.
+    auto emit = [&](uint32_t len, uint8_t op) {
+        for (uint32_t k = lane; k < len; k += 32)
+            if (cnt + k < cap) slot[cap - 1 - cnt - k] = op;
+        cnt = min(cap, cnt + len);
+    };
     uint32_t i = brow, j = bcol;
-    int state = 0;
+    uint32_t state = 0;
     int32_t v = bs;  // local mode: the value of the cell the walk stands on (H, E or F by state)
     const int32_t go = P.go, ge = P.ge;
-    // Each iteration emits an operation or changes state once between two operations, so the
-    // walk ends within 2 (m + n) + 2 iterations.
-    for (uint64_t it = 0; it < 2 * cap + 4; ++it) {
+    // Each iteration emits an operation, so the walk ends within m + n + 1 iterations.
+    for (uint64_t it = 0; it < cap + 2; ++it) {
         if (i == 0 || j == 0) {
             // Border (src/align.rs:366-383): nothing but a penalised border gap remains. The E
             // and F states always return to H before reaching a border row or column.
             if constexpr (!F::local && !F::top_free) {
-                if (i == 0)
-                    while (j > 0 && cnt < cap) {
-                        slot[cap - 1 - cnt++] = 3;
-                        --j;
-                    }
+                if (i == 0) {
+                    emit(j, 3);
+                    j = 0;
+                }
             }
             if constexpr (!F::local && !F::left_free) {
-                if (j == 0)
-                    while (i > 0 && cnt < cap) {
-                        slot[cap - 1 - cnt++] = 2;
-                        --i;
-                    }
+                if (j == 0) {
+                    emit(i, 2);
+                    i = 0;
+                }
             }
             break;
         }
-        if (F::local && state == 0 && v == 0) break;  // local && H == 0 (src/align.rs:362-365)
-        const uint32_t code = tb_code(D, r_log2, pass_stride, n, i, j);
+        uint32_t code = 0;
+        bool known = false;  // `code` is the code of cell (i, j)
         if (state == 0) {
-            const uint32_t src = code & 3u;
-            if (src == 0u) {
-                const uint32_t a = qs[i - 1], b = ts[j - 1];
-                if (cnt < cap) slot[cap - 1 - cnt++] = a == b ? 0 : 1;
-                if (F::local) v -= P.matrix[a * P.al + b];  // H(i-1, j-1) = H(i, j) - sub
-                --i;
-                --j;
-                continue;
+            const uint32_t len = min(32u, min(i, j));  // cells before the border
+            const bool in = lane < len;
+            const uint32_t c = in ? tb_code(D, r_log2, pass_stride, n, i - lane, j - lane) : 1u;
+            const uint32_t a = in ? qs[i - 1 - lane] : 0u, b = in ? ts[j - 1 - lane] : 0u;
+            // Lanes [0, run) step diagonally.
+            const uint32_t stop = ~__ballot_sync(0xffffffffu, (c & 3u) == 0u);
+            uint32_t run = stop ? (uint32_t)__ffs(stop) - 1 : 32u;
+            bool at_zero = false;
+            if constexpr (F::local) {
+                // H(i-1, j-1) = H(i, j) - sub: the values of lanes [0, run] (src/align.rs:362-365: stop at H == 0).
+                const int32_t sub = in ? P.matrix[a * P.al + b] : 0;
+                int32_t sum = sub;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int32_t x = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= (uint32_t)o) sum += x;
+                }
+                const uint32_t zero = __ballot_sync(0xffffffffu, lane <= run && v - (sum - sub) == 0);
+                if (zero) {
+                    run = (uint32_t)__ffs(zero) - 1;
+                    at_zero = true;
+                }
+                const int32_t taken = __shfl_sync(0xffffffffu, sum, (run + 31) & 31);
+                if (run > 0) v -= taken;
             }
-            state = (int)src;  // the gap step below reads the same cell's code (E or F = H here)
+            if (lane < run && cnt + lane < cap) slot[cap - 1 - cnt - lane] = a == b ? 0 : 1;
+            cnt = min(cap, cnt + run);
+            i -= run;
+            j -= run;
+            if (at_zero) break;
+            if (run == len) continue;  // the border, or 32 cells
+            code = __shfl_sync(0xffffffffu, c, run);
+            known = true;
+            state = code & 3u;  // the gap step reads the same cell's code (E or F = H here)
         }
-        if (state == 1) {
-            if (cnt < cap) slot[cap - 1 - cnt++] = 3;
-            --j;
-            if (!(code & 4u)) {
-                state = 0;
-                if (F::local) v += go;  // H(i, j - 1) = E(i, j) + go
-            } else if (F::local) {
-                v += ge;  // E(i, j - 1) = E(i, j) + ge
-            }
-        } else {
-            if (cnt < cap) slot[cap - 1 - cnt++] = 2;
-            --i;
-            if (!(code & 8u)) {
-                state = 0;
-                if (F::local) v += go;  // H(i - 1, j) = F(i, j) + go
-            } else if (F::local) {
-                v += ge;  // F(i - 1, j) = F(i, j) + ge
-            }
+        const bool left = state == 1;
+        const uint32_t flag = left ? 4u : 8u;
+        const uint32_t len = min(32u, left ? j : i);
+        uint32_t run = 0;  // cells of the gap that extend
+        if (!known || (code & flag)) {
+            const uint32_t c = lane < len ? tb_code(D, r_log2, pass_stride, n, left ? i : i - lane, left ? j - lane : j) : 0u;
+            const uint32_t stop = ~__ballot_sync(0xffffffffu, (c & flag) != 0u);
+            run = stop ? (uint32_t)__ffs(stop) - 1 : 32u;
         }
+        const bool closed = run < len;
+        const uint32_t steps = closed ? run + 1 : len;
+        emit(steps, left ? 3 : 2);
+        if (left) j -= steps;
+        else i -= steps;
+        // E(i, j-1) = E(i, j) + ge while the gap extends, H(i, j-1) = E(i, j) + go where it opens.
+        if (F::local) v += (int32_t)run * ge + (closed ? go : 0);
+        if (closed) state = 0;
     }
+    if (lane != 0) return;
     hy_alignment a;
     a.score = bs;
     a.query_start = i;
@@ -874,13 +907,12 @@ static cudaError_t launch_fill(uint32_t R, const TbParams &p, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// The walk is one thread per pair and bound by the latency of its dependent code loads: small
-// blocks spread the walkers over every SM.
+// Small blocks spread the walking warps over every SM.
 constexpr int TB_WALK_BLOCK = 64;
 
 template <int MODE>
 static cudaError_t launch_walk(const TbParams &p, cudaStream_t st) {
-    tb_walk_kernel<MODE><<<(p.n_pairs + TB_WALK_BLOCK - 1) / TB_WALK_BLOCK, TB_WALK_BLOCK, 0, st>>>(p);
+    tb_walk_kernel<MODE><<<(uint32_t)(((uint64_t)p.n_pairs * 32 + TB_WALK_BLOCK - 1) / TB_WALK_BLOCK), TB_WALK_BLOCK, 0, st>>>(p);
     return cudaGetLastError();
 }
 
