@@ -807,7 +807,31 @@ static void tb_plan(uint64_t m, uint64_t max_n, uint32_t n_pairs, uint32_t *R, b
     *R = *stripes ? TB_STRIPE_R : tb_rows(m, max_n);
 }
 
+// Of many pairs, the longest whose chain of passes on one warp would outlast the rest also run on
+// the stripe kernel, beside the fill: a step of R rows takes a lone warp TB_STEP_US * (R + 6), one
+// of a stripe TB_STRIPE_STEP_US, and the fill computes TB_FILL_CELLS padded cells a microsecond with
+// every SM busy (measured). A chain shorter than a third of the fill's busy time hides in it, since the
+// longest pairs start first. TB_MAX_STRIPES: a stripe's warp a scheduler. (A query of 600 against 10,000
+// protein targets, 40 to some 7,000 residues: fill 8.6 to 5.6 ms.)
+constexpr double TB_STEP_US = 0.03, TB_STRIPE_STEP_US = 0.4, TB_FILL_CELLS = 775e3;
+constexpr uint32_t TB_MAX_STRIPES = 148 * 4;
+
 static uint64_t tb_passes(uint64_t m, uint32_t R) { return std::max<uint64_t>(1, (m + 32 * R - 1) / (32 * R)); }
+
+// How many of the longest pairs (lengths n[0] >= n[1] >= ...) leave the fill of R rows per lane.
+static uint32_t tb_stripe_pairs(uint64_t m, uint32_t R, const std::vector<uint64_t> &n) {
+    const uint64_t S = tb_passes(m, TB_STRIPE_R), passes = tb_passes(m, R);
+    if (m == 0 || S < 2) return 0;
+    double cells = 0;
+    for (uint64_t x : n) cells += (double)(x + 31) * (double)(passes * 32 * R);
+    uint32_t k = 0;
+    for (; k < n.size() && n[k] > 0 && (k + 1) * S <= TB_MAX_STRIPES; ++k) {
+        const double chain = (double)passes * (double)(n[k] + 31) * TB_STEP_US * (R + 6);
+        const double striped = (double)(n[k] + 31 + 63 * (S - 1)) * TB_STRIPE_STEP_US;
+        if (chain < cells / TB_FILL_CELLS / 3 || striped > 0.7 * chain) break;
+    }
+    return k;
+}
 
 static uint64_t tb_dir_bytes(uint64_t m, uint64_t n, uint32_t R) {
     if (m == 0 || n == 0) return 0;
@@ -846,6 +870,7 @@ struct TbContext {
     int device = -1;
     cudaStream_t stream = nullptr;    // fills, then the copies back (the caller's stream)
     cudaStream_t stream_b = nullptr;  // walks and compaction, overlapping the next chunk's fill
+    cudaStream_t stream_s = nullptr;  // the stripes of the longest pairs, beside the fill of the others
     bool own_stream = false;
     uint8_t *d_q = nullptr, *d_t = nullptr, *d_ops = nullptr, *d_ops_out = nullptr;
     uint8_t *d_dir[2] = {nullptr, nullptr};  // codes of two chunks in flight
@@ -876,6 +901,7 @@ struct TbContext {
     ~TbContext() {
         if (stream) cudaStreamSynchronize(stream);
         if (stream_b) cudaStreamSynchronize(stream_b);
+        if (stream_s) cudaStreamSynchronize(stream_s);
         for (cudaEvent_t e : ev) cudaEventDestroy(e);
         for (void *p : {(void *)d_q, (void *)d_t, (void *)d_dir[0], (void *)d_dir[1], (void *)d_ops,
                         (void *)d_ops_out, (void *)d_prof, (void *)d_matrix, (void *)d_bnd, (void *)d_pairs,
@@ -885,6 +911,7 @@ struct TbContext {
                         (void *)h_first, (void *)h_stage})
             cudaFreeHost(p);
         if (stream_b) cudaStreamDestroy(stream_b);
+        if (stream_s) cudaStreamDestroy(stream_s);
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
 };
@@ -1024,11 +1051,24 @@ static hy_status tb_run(TbContext &ctx, const TbRun &run, const uint32_t *idx, u
     }
     std::vector<uint32_t> chunk_at{0};
     uint64_t dir_max = 0, bnd_max = 0, dir = 0, bnd = 0;
-    const uint32_t per_pair = run.stripes ? (uint32_t)tb_passes(run.m, run.R) : 1u;
+    const uint32_t per_pair = (uint32_t)tb_passes(run.m, TB_STRIPE_R);  // stripes of a striped pair
+    uint32_t n_striped = n_idx;                                          // pairs [0, n_striped) of the order
+    if (!run.stripes) {
+        std::vector<uint64_t> lens(n_idx);
+        for (uint32_t x = 0; x < n_idx; ++x) lens[x] = t_len(idx[order[x]]);
+        n_striped = tb_stripe_pairs(run.m, run.R, lens);
+    }
+    if (n_striped > 0 && n_striped < n_idx && !ctx.stream_s) {
+        int lo = 0, hi = 0;
+        TB_CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+        TB_CK(cudaStreamCreateWithPriority(&ctx.stream_s, cudaStreamNonBlocking, hi));
+    }
     for (uint32_t x = 0; x < n_idx; ++x) {
+        const bool striped = x < n_striped;
+        const uint32_t R = striped ? TB_STRIPE_R : run.R;
         const uint32_t s = order[x], k = idx[s];
         const uint64_t n = t_len(k);
-        const uint64_t d = align16(tb_dir_bytes(run.m, n, run.R));
+        const uint64_t d = align16(tb_dir_bytes(run.m, n, R));
         if (x > chunk_at.back() && dir + d > TB_CHUNK_BYTES) {
             chunk_at.push_back(x);
             dir = bnd = 0;
@@ -1041,14 +1081,14 @@ static hy_status tb_run(TbContext &ctx, const TbRun &run, const uint32_t *idx, u
         pp.n = (uint32_t)n;
         pp.m_pad = run.m_pad;
         pp.slot = s;
-        pp.rows = run.R;
-        pp.n_ends = per_pair;
-        pp.ends_off = run.stripes ? (uint64_t)x * per_pair : s;
+        pp.rows = R;
+        pp.n_ends = striped ? per_pair : 1;
+        pp.ends_off = striped ? (uint64_t)x * per_pair : (uint64_t)n_striped * per_pair + x - n_striped;
         pp.dir_off = dir;
         pp.bnd_off = bnd;
         pp.ops_off = ops_at[s];
         dir += d;
-        bnd += run.stripes ? (uint64_t)(per_pair - 1) * (n + 1) : n + 1;
+        bnd += striped ? (uint64_t)(per_pair - 1) * (n + 1) : n + 1;
         dir_max = std::max(dir_max, dir);
         bnd_max = std::max(bnd_max, bnd);
         ctx.cells += (double)run.m * (double)n;
@@ -1061,22 +1101,22 @@ static hy_status tb_run(TbContext &ctx, const TbRun &run, const uint32_t *idx, u
     TB_CK(grow(ctx.d_bnd, ctx.c_bnd, sizeof(int2) * bnd_max));
     TB_CK(grow(ctx.d_ops, ctx.c_ops, oo));
     TB_CK(grow(ctx.d_ops_out, ctx.c_ops_out, oo));
-    TB_CK(grow(ctx.d_ends, ctx.c_ends, sizeof(TbEnd) * n_idx * per_pair));
-    if (run.stripes) {
-        TB_CK(grow(ctx.d_prog, ctx.c_prog, sizeof(uint32_t) * (uint64_t)n_idx * per_pair + 16));
+    TB_CK(grow(ctx.d_ends, ctx.c_ends, sizeof(TbEnd) * ((uint64_t)n_striped * per_pair + n_idx - n_striped)));
+    if (n_striped > 0) {
+        TB_CK(grow(ctx.d_prog, ctx.c_prog, sizeof(uint32_t) * (uint64_t)n_striped * per_pair + 16));
         TB_CK(cudaMemsetAsync(ctx.d_prog, 0, 16, ctx.stream));  // the error flag sits in front
-        // Every pair has per_pair stripes: chunk-local pair x owns [x, x + 1) * per_pair.
-        TB_CK(grow(ctx.d_first, ctx.c_first, sizeof(uint32_t) * (n_idx + 1)));
-        TB_CK(grow_pinned(ctx.h_first, ctx.ch_first, sizeof(uint32_t) * (n_idx + 1)));
-        for (uint32_t x = 0; x <= n_idx; ++x) ctx.h_first[x] = x * per_pair;
-        TB_CK(cudaMemcpyAsync(ctx.d_first, ctx.h_first, sizeof(uint32_t) * (n_idx + 1), cudaMemcpyHostToDevice,
+        // Every striped pair has per_pair stripes: chunk-local pair x owns [x, x + 1) * per_pair.
+        TB_CK(grow(ctx.d_first, ctx.c_first, sizeof(uint32_t) * (n_striped + 1)));
+        TB_CK(grow_pinned(ctx.h_first, ctx.ch_first, sizeof(uint32_t) * (n_striped + 1)));
+        for (uint32_t x = 0; x <= n_striped; ++x) ctx.h_first[x] = x * per_pair;
+        TB_CK(cudaMemcpyAsync(ctx.d_first, ctx.h_first, sizeof(uint32_t) * (n_striped + 1), cudaMemcpyHostToDevice,
                               ctx.stream));
     }
     TB_CK(grow(ctx.d_out, ctx.c_out, sizeof(hy_alignment) * n_idx));
     TB_CK(grow(ctx.d_total, ctx.c_total, 16));
     TB_CK(grow_pinned(ctx.h_out, ctx.ch_out, sizeof(hy_alignment) * n_idx));
     TB_CK(grow_pinned(ctx.h_total, ctx.ch_total, 16));
-    while (ctx.ev.size() < 4 * n_chunks + 2) {
+    while (ctx.ev.size() < 5 * n_chunks + 2) {
         cudaEvent_t e;
         TB_CK(cudaEventCreate(&e));
         ctx.ev.push_back(e);
@@ -1106,17 +1146,31 @@ static hy_status tb_run(TbContext &ctx, const TbRun &run, const uint32_t *idx, u
         p.dir = ctx.d_dir[c & 1];
         if (c >= 2) TB_CK(cudaStreamWaitEvent(ctx.stream, ctx.ev[4 * (c - 2) + 3], 0));
         TB_CK(cudaEventRecord(e[0], ctx.stream));
-        if (run.m > 0 && run.stripes) {
-            const uint32_t n_str = p.n_pairs * per_pair;
+        // The chunk's striped pairs come first; alone they take `stream`, else a stream beside the fill's.
+        const uint32_t n_str_pairs = run.m > 0 && n_striped > chunk_at[c] ? std::min(n_striped, chunk_at[c + 1]) - chunk_at[c] : 0;
+        const bool beside = n_str_pairs > 0 && n_str_pairs < p.n_pairs;
+        cudaEvent_t e_str = ctx.ev[4 * n_chunks + 2 + c];
+        if (n_str_pairs > 0) {
+            const cudaStream_t st = beside ? ctx.stream_s : ctx.stream;
+            if (beside) TB_CK(cudaStreamWaitEvent(st, e[0], 0));
+            const uint32_t n_str = n_str_pairs * per_pair;
+            TbParams ps = p;
+            ps.n_pairs = n_str_pairs;
             TbStripes S{ctx.d_first, n_str, tb_stripe_smem_al(run.al), ctx.d_bnd, ctx.d_prog + 4, (int *)ctx.d_prog,
                         tb_spin_limit()};
-            TB_CK(cudaMemsetAsync(S.prog, 0, sizeof(uint32_t) * n_str, ctx.stream));
-            TB_CK(dispatch_stripes(run.mode, true, p, S, ctx.stream, ctx.device));
+            TB_CK(cudaMemsetAsync(S.prog, 0, sizeof(uint32_t) * n_str, st));
+            TB_CK(dispatch_stripes(run.mode, true, ps, S, st, ctx.device));
+            if (beside) TB_CK(cudaEventRecord(e_str, st));
             ctx.launches += 2;
-        } else if (run.m > 0) {
-            TB_CK(dispatch_fill(run.mode, run.R, p, ctx.stream));
+        }
+        if (run.m > 0 && n_str_pairs < p.n_pairs) {
+            TbParams pf = p;
+            pf.pairs += n_str_pairs;
+            pf.n_pairs -= n_str_pairs;
+            TB_CK(dispatch_fill(run.mode, run.R, pf, ctx.stream));
             ++ctx.launches;
         }
+        if (beside) TB_CK(cudaStreamWaitEvent(ctx.stream, e_str, 0));
         TB_CK(cudaEventRecord(e[1], ctx.stream));
         TB_CK(cudaStreamWaitEvent(ctx.stream_b, e[1], 0));
         TB_CK(cudaEventRecord(e[2], ctx.stream_b));
@@ -1137,9 +1191,9 @@ static hy_status tb_run(TbContext &ctx, const TbRun &run, const uint32_t *idx, u
     TB_CK(cudaStreamWaitEvent(ctx.stream, e_end, 0));
     TB_CK(cudaMemcpyAsync(ctx.h_out, ctx.d_out, sizeof(hy_alignment) * n_idx, cudaMemcpyDeviceToHost, ctx.stream));
     TB_CK(cudaMemcpyAsync(ctx.h_total, ctx.d_total, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx.stream));
-    if (run.stripes) TB_CK(cudaMemcpyAsync(ctx.h_total + 1, ctx.d_prog, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
+    if (n_striped > 0) TB_CK(cudaMemcpyAsync(ctx.h_total + 1, ctx.d_prog, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
     TB_CK(cudaStreamSynchronize(ctx.stream));
-    if (run.stripes && *(const uint32_t *)(ctx.h_total + 1)) return fail(HY_ERR_TIMEOUT);
+    if (n_striped > 0 && *(const uint32_t *)(ctx.h_total + 1)) return fail(HY_ERR_TIMEOUT);
     const uint64_t total = *ctx.h_total;
     if (ops_direct) {
         if (total) TB_CK(cudaMemcpyAsync(ops_direct, ctx.d_ops_out, total, cudaMemcpyDeviceToHost, ctx.stream));
