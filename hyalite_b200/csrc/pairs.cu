@@ -35,6 +35,8 @@ namespace hy {
 
 constexpr int PAIR_G = 8;
 constexpr int PAIR_R32 = 16;
+constexpr int PAIR_WIDE_G = 32;  // lanes of the wide form: a warp an item
+constexpr int PAIR_WIDE_GPB = 2;  // its items a block: small blocks, so that a long item holds little of an SM
 constexpr size_t PAIR_SMEM_LIMIT = 200 * 1024;
 // Largest global scratch for group profiles that do not fit in shared memory, per launch.
 constexpr size_t PAIR_GPROF_BYTES = 256ull << 20;
@@ -126,6 +128,9 @@ struct PairsContext {
     cudaStream_t stream = nullptr;       // packing kernels, pair kernels, results
     cudaStream_t copy_stream = nullptr;  // host-to-device copies of the chunks
     cudaStream_t d2h_stream = nullptr;   // position maxima: each chunk's column maxima back
+    cudaStream_t side_stream = nullptr;  // a chunk's wide items, beside its other items
+    cudaStream_t long_stream = nullptr;  // the stripe kernel's long pairs, beside the chunks
+    cudaEvent_t ev_fork = nullptr, ev_side = nullptr, ev_long = nullptr;
     std::vector<cudaEvent_t> ev;         // around each chunk's device work, then its copy back
     cudaEvent_t slot_ev[PAIR_SLOTS] = {};
     struct Buf {
@@ -148,6 +153,10 @@ struct PairsContext {
         if (stream) cudaStreamDestroy(stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
         if (d2h_stream) cudaStreamDestroy(d2h_stream);
+        if (side_stream) cudaStreamDestroy(side_stream);
+        if (long_stream) cudaStreamDestroy(long_stream);
+        for (cudaEvent_t e : {ev_fork, ev_side, ev_long})
+            if (e) cudaEventDestroy(e);
     }
     cudaError_t get_pinned(int slot, size_t bytes, void **out) {
         bytes = std::max<size_t>(bytes, 16);
@@ -162,13 +171,14 @@ struct PairsContext {
         *out = pinned[slot].p;
         return cudaSuccess;
     }
-    // Device buffer of at least `bytes`. Growing a buffer the compute stream may still be reading
-    // first waits for that stream.
+    // Device buffer of at least `bytes`. Growing a buffer the compute streams may still be reading
+    // first waits for them.
     cudaError_t get(int slot, size_t bytes, void **out) {
         bytes = std::max<size_t>(bytes, 16);
         if (b[slot].n < bytes) {
             if (stream) {
                 cudaError_t e = cudaStreamSynchronize(stream);
+                if (e == cudaSuccess && side_stream) e = cudaStreamSynchronize(side_stream);
                 if (e != cudaSuccess) return e;
             }
             hy::dev_free(b[slot].p);
@@ -332,8 +342,10 @@ static cudaError_t launch_pairs_gprof(int mode, bool ends, const PairParams &p, 
 template <class A, int G, int R>
 static cudaError_t launch_pairs(int mode, bool ends, const PairParams &p, int blocks, int threads,
                                 size_t smem, cudaStream_t st) {
-    if (p.gprof) return launch_pairs_gprof<A, G, R>(mode, ends, p, blocks, threads, st);
-    if (p.colmax) return launch_pairs_mode<A, G, R, MODE_SW, false, false, true>(p, blocks, threads, smem, st);
+    if constexpr (G != PAIR_WIDE_G)
+        if (p.gprof) return launch_pairs_gprof<A, G, R>(mode, ends, p, blocks, threads, st);
+    if constexpr (G != PAIR_WIDE_G)
+        if (p.colmax) return launch_pairs_mode<A, G, R, MODE_SW, false, false, true>(p, blocks, threads, smem, st);
 #define HY_MODE_CASE(M)                                                                        \
     case M:                                                                                    \
         return ends ? launch_pairs_mode<A, G, R, M, true, false>(p, blocks, threads, smem, st) \
@@ -352,7 +364,10 @@ static cudaError_t launch_pairs(int mode, bool ends, const PairParams &p, int bl
 template <class A, int G>
 static cudaError_t launch_pairs_rows(int rows, int mode, bool ends, const PairParams &p, int blocks,
                                      int threads, size_t smem, cudaStream_t st) {
-    if constexpr (A::NH == 2) {
+    if constexpr (G == PAIR_WIDE_G) {
+        if (rows == 4) return launch_pairs<A, G, 4>(mode, ends, p, blocks, threads, smem, st);
+        return launch_pairs<A, G, 8>(mode, ends, p, blocks, threads, smem, st);
+    } else if constexpr (A::NH == 2) {
         switch (rows) {
         case 8: return launch_pairs<A, G, 8>(mode, ends, p, blocks, threads, smem, st);
         case 12: return launch_pairs<A, G, 12>(mode, ends, p, blocks, threads, smem, st);
@@ -590,12 +605,61 @@ static size_t pack_items(PairsHost &hs, const uint32_t *order, const uint64_t *k
     return n_items;
 }
 
+// Rows per lane of the wide form: one pass of 128 rows, else passes of 256.
+static int pair_wide_rows(uint64_t q) { return q <= 128 ? 4 : 8; }
+
+// How many of one chunk's int16x2 items, sorted longest query first, take the wide form: 32 lanes an
+// item, so a chain a third to a quarter as long, and no columns padded to the longest of four items that
+// share a warp; but fewer rows share a step's fixed work. The split, at one of 16 places, is the one of
+// least estimated time: the warp-instructions of both forms (a step of R rows 50 + 9 R) over 148 SMs of
+// 4 schedulers at 1.46 cycles, or the longest chain at 2.2. (5,000
+// protein pairs of all lengths: 6.2 ms of narrow kernels, 11.5 ms a call; so, with the long pairs' stripes
+// beside them, 5.4. 150-base reads keep the narrow form.)
+static size_t pair_wide_split(const ItemMeta *meta, const uint32_t *qlen, size_t n, int32_t al) {
+    constexpr size_t PARTS = 16;
+    const size_t per = ((n + PARTS - 1) / PARTS + 3) / 4 * 4;  // whole warps of the narrow form
+    double work[2][PARTS] = {}, chain[2][PARTS] = {};
+    uint32_t q_last = 0;
+    int r = 8;
+    for (size_t b = 0; b * per < n; ++b) {
+        for (size_t i = b * per; i < std::min(n, (b + 1) * per); i += 4) {
+            uint32_t w = 0, q = 0;
+            const size_t e = std::min(n, i + 4);
+            for (size_t k = i; k < e; ++k) {
+                w = std::max(w, meta[k].w);
+                q = std::max(q, qlen[k]);
+                const int rw = pair_wide_rows(qlen[k]);
+                const double c = (double)((qlen[k] + 32 * rw - 1) / (32 * rw)) * (meta[k].w + 31.0) * (50.0 + 9.0 * rw);
+                work[1][b] += c;
+                chain[1][b] = std::max(chain[1][b], c);
+            }
+            if (q != q_last) r = pair_rows(q, al), q_last = q;
+            const double c = (double)((q + 8 * r - 1) / (8 * r)) * (w + 7.0) * (50.0 + 9.0 * r);
+            work[0][b] += c;
+            chain[0][b] = std::max(chain[0][b], c);
+        }
+    }
+    size_t best = 0;
+    double best_t = 1e300;
+    for (size_t s = 0; s <= PARTS; ++s) {
+        double w = 0, c = 0;
+        for (size_t b = 0; b < PARTS; ++b) {
+            w += work[b < s][b];
+            c = std::max(c, chain[b < s][b]);
+        }
+        const double t = std::max(w / (148 * 4) * 1.46, c * 2.2);
+        if (t < 0.95 * best_t) best_t = t, best = std::min(n, s * per);
+    }
+    return best;
+}
+
 // Packs and aligns one chunk's items of one lane arithmetic: the packing kernel, then one launch
-// per run of items with the same rows per lane (items are sorted by query length). Items
+// per run of items with the same rows per lane (items are sorted by query length; the wide items on
+// the side stream, joined back at the end). meta (host): the chunk's items. Items
 // [ib, ib + n_items) of the call; qlen (host) their query lengths; cols the chunk's columns.
 template <class A, int G>
 static hy_status run_items(PairsContext &ctx, PairParams p, int res_slot, int bnd_slot,
-                           const uint32_t *qlen, size_t ib, size_t n_items, uint64_t cols,
+                           const uint32_t *qlen, const ItemMeta *meta, size_t ib, size_t n_items, uint64_t cols,
                            const uint64_t *d_qoff, const uint64_t *d_toff, uint8_t *d_q,
                            const uint8_t *d_t, uint32_t *d_bad, int mode, bool ends) {
     if (n_items == 0) return fail(HY_OK);
@@ -612,8 +676,14 @@ static hy_status run_items(PairsContext &ctx, PairParams p, int res_slot, int bn
     }
     // Rows per lane of each run of equal query lengths.
     auto rows_of = [&](uint32_t q) { return two ? pair_rows(q, p.al) : PAIR_R32; };
+    // The wide items [0, n_wide): not the column-maxima form, nor a large alphabet.
+    size_t n_wide = 0;
+    const size_t wide_bytes = (size_t)(p.al + 1) * PAIR_WIDE_G * profile_row_bytes<A>();  // a row per lane
+    if (two && !p.colmax && PAIR_WIDE_GPB * 8 * wide_bytes <= PAIR_SMEM_LIMIT)
+        n_wide = pair_wide_split(meta, qlen, n_items, p.al);
     bool multipass = false;
-    for (size_t i = 0; i < n_items;) {
+    for (size_t i = 0; i < n_wide; ++i) multipass = multipass || qlen[i] > (uint32_t)(PAIR_WIDE_G * pair_wide_rows(qlen[i]));
+    for (size_t i = n_wide; i < n_items;) {
         size_t j = i;
         while (j < n_items && qlen[j] == qlen[i]) ++j;
         multipass = multipass || qlen[i] > (uint32_t)(G * rows_of(qlen[i]));
@@ -624,7 +694,26 @@ static hy_status run_items(PairsContext &ctx, PairParams p, int res_slot, int bn
     p.res = d_res;
     p.boundary = d_bnd;
     p.gprof = nullptr;
-    for (size_t i0 = 0; i0 < n_items;) {
+    if constexpr (two) {
+        if (n_wide > 0) {
+            HY_CK(cudaEventRecord(ctx.ev_fork, ctx.stream));
+            HY_CK(cudaStreamWaitEvent(ctx.side_stream, ctx.ev_fork, 0));
+            for (size_t i0 = 0; i0 < n_wide;) {
+                const int r = pair_wide_rows(qlen[i0]);
+                size_t i1 = i0;
+                while (i1 < n_wide && pair_wide_rows(qlen[i1]) == r) ++i1;
+                p.group_bytes = (uint32_t)(wide_bytes * r);
+                p.item_base = (uint32_t)(ib + i0);
+                p.n_items = (uint32_t)(ib + i1);
+                const int blocks = (int)((i1 - i0 + PAIR_WIDE_GPB - 1) / PAIR_WIDE_GPB);
+                HY_CK((launch_pairs_rows<A, PAIR_WIDE_G>(r, mode, ends, p, blocks, PAIR_WIDE_GPB * PAIR_WIDE_G,
+                                                         PAIR_WIDE_GPB * wide_bytes * r, ctx.side_stream)));
+                i0 = i1;
+            }
+            HY_CK(cudaEventRecord(ctx.ev_side, ctx.side_stream));
+        }
+    }
+    for (size_t i0 = n_wide; i0 < n_items;) {
         const int r = rows_of(qlen[i0]);
         size_t i1 = i0;
         while (i1 < n_items && (qlen[i1] == qlen[i0] || rows_of(qlen[i1]) == r)) ++i1;
@@ -657,6 +746,7 @@ static hy_status run_items(PairsContext &ctx, PairParams p, int res_slot, int bn
         }
         i0 = i1;
     }
+    if (n_wide > 0) HY_CK(cudaStreamWaitEvent(ctx.stream, ctx.ev_side, 0));
     return fail(HY_OK);
 }
 
@@ -859,6 +949,10 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             HY_CK(cudaStreamCreateWithFlags(&ctx.stream, cudaStreamNonBlocking));
             HY_CK(cudaStreamCreateWithFlags(&ctx.copy_stream, cudaStreamNonBlocking));
             HY_CK(cudaStreamCreateWithFlags(&ctx.d2h_stream, cudaStreamNonBlocking));
+            HY_CK(cudaStreamCreateWithFlags(&ctx.side_stream, cudaStreamNonBlocking));
+            HY_CK(cudaStreamCreateWithFlags(&ctx.long_stream, cudaStreamNonBlocking));
+            for (cudaEvent_t *e : {&ctx.ev_fork, &ctx.ev_side, &ctx.ev_long})
+                HY_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
             for (cudaEvent_t &e : ctx.slot_ev) HY_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
         const uint64_t L = n_len;
@@ -945,6 +1039,13 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
         HY_CK(cudaMemsetAsync(d_bad, 0xff, sizeof(uint32_t), ctx.stream));
         HY_CK(cudaMemcpyAsync(d_matrix, matrix, sizeof(int32_t) * alphabet_len * alphabet_len,
                               cudaMemcpyHostToDevice, ctx.stream));
+        // The long pairs run beside the chunks, on a stream that waits for the matrix and the queries (with
+        // column maxima after the chunks, which zero them).
+        const cudaStream_t long_st = posmax ? ctx.stream : ctx.long_stream;
+        if (!run_long.empty() && !posmax) {
+            HY_CK(cudaEventRecord(ctx.ev_long, ctx.stream));
+            HY_CK(cudaStreamWaitEvent(long_st, ctx.ev_long, 0));
+        }
         uint64_t ib[2] = {0, 0};
         // Declared before the drainer, whose thread reads it: locals are destroyed in reverse
         // order, so the thread is joined (on any early return) before this vector goes away.
@@ -1070,11 +1171,11 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             HY_CK(cudaStreamWaitEvent(ctx.stream, ctx.slot_ev[cs.s], 0));
             if (posmax && tb) HY_CK(cudaMemsetAsync(d_colmax + t_off[a], 0, sizeof(int32_t) * tb, ctx.stream));
             HY_CK(cudaEventRecord(ctx.ev[2 * c], ctx.stream));
-            hy_status s2 = run_items<Pair16H, PAIR_G>(ctx, pp[0], PS_RES16, PS_BND16, cs.qlen[0], ib[0], cs.n_items[0],
+            hy_status s2 = run_items<Pair16H, PAIR_G>(ctx, pp[0], PS_RES16, PS_BND16, cs.qlen[0], cs.s_meta[0], ib[0], cs.n_items[0],
                                                       cs.cols[0], (const uint64_t *)d_qoff, (const uint64_t *)d_toff,
                                                       (uint8_t *)d_q, (const uint8_t *)d_t, d_bad, mode, ends);
             if (s2 != HY_OK) return s2;
-            s2 = run_items<Single32, PAIR_G>(ctx, pp[1], PS_RES32, PS_BND32, cs.qlen[1], ib[1], cs.n_items[1],
+            s2 = run_items<Single32, PAIR_G>(ctx, pp[1], PS_RES32, PS_BND32, cs.qlen[1], cs.s_meta[1], ib[1], cs.n_items[1],
                                              cs.cols[1], (const uint64_t *)d_qoff, (const uint64_t *)d_toff,
                                              (uint8_t *)d_q, (const uint8_t *)d_t, d_bad, mode, ends);
             if (s2 != HY_OK) return s2;
@@ -1126,8 +1227,11 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             have_pend = true;
         }
         if (have_pend && (st = flush()) != HY_OK) return st;
-        // The long pairs, once every chunk's queries are on the device (the compute stream has
-        // waited for each chunk's copies).
+        // The long pairs, once every chunk's queries are on the device.
+        if (!run_long.empty() && !posmax) {
+            HY_CK(cudaEventRecord(ctx.ev_long, ctx.copy_stream));
+            HY_CK(cudaStreamWaitEvent(long_st, ctx.ev_long, 0));
+        }
         if (run_long.size() == 1 && !posmax &&
             band_long_pair_fits(q_off[run_long[0] + 1] - q_off[run_long[0]], alphabet_len)) {
             // One long pair (align_pair's single-pair path) whose passes fit one round: the band
@@ -1137,13 +1241,13 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             const uint32_t k = run_long[0];
             st = band_long_pair((const uint8_t *)d_q + q_off[k], q_off[k + 1] - q_off[k], t_res + t_off[k],
                                 t_off[k + 1] - t_off[k], (const int32_t *)d_matrix, alphabet_len, gap_open,
-                                gap_ext, mode, ctx.stream, k, d_scores, d_qend, d_tend, &ctx.kernel_ms);
+                                gap_ext, mode, long_st, k, d_scores, d_qend, d_tend, &ctx.kernel_ms);
             if (st != HY_OK) return st;
         } else if (!run_long.empty()) {
             const TbColmaxOut cmx{d_colmax, pc.score2 ? d_s2 : nullptr, max_e, pc.min_score};
             st = tb_long_pair_scores(q_res, q_off, t_res, t_off, run_long, (const uint8_t *)d_q,
                                      (const int32_t *)d_matrix, alphabet_len, gap_open, gap_ext, mode,
-                                     ctx.stream, d_scores, d_qend, d_tend, &ctx.kernel_ms,
+                                     long_st, d_scores, d_qend, d_tend, &ctx.kernel_ms,
                                      posmax ? &cmx : nullptr);
             if (st != HY_OK) return st;
         }
