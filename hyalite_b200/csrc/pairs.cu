@@ -1236,8 +1236,8 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             band_long_pair_fits(q_off[run_long[0] + 1] - q_off[run_long[0]], alphabet_len)) {
             // One long pair (align_pair's single-pair path) whose passes fit one round: the band
             // kernel, its passes on the warps of one block or of a cluster, ends tracked in the
-            // same sweep (measured 2000 x 2000 0.55 ms, 5000 x 5000 1.6 ms against the stripe
-            // kernel's 0.97 and 2.5 ms; at 20,000 query rows, two rounds, the stripes are faster).
+            // same sweep (measured kernels: 2000 x 2000 0.23 ms, 5000 x 5000 0.67 ms against the
+            // stripe kernel's 0.97 and 2.5 ms; at 20,000 query rows, two rounds, the stripes are faster).
             const uint32_t k = run_long[0];
             st = band_long_pair((const uint8_t *)d_q + q_off[k], q_off[k + 1] - q_off[k], t_res + t_off[k],
                                 t_off[k + 1] - t_off[k], (const int32_t *)d_matrix, alphabet_len, gap_open,
