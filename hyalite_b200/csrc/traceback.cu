@@ -1145,20 +1145,26 @@ static hy_status tb_run(TbContext &ctx, const TbRun &run, const uint32_t *idx, u
         p.n_pairs = chunk_at[c + 1] - chunk_at[c];
         p.dir = ctx.d_dir[c & 1];
         if (c >= 2) TB_CK(cudaStreamWaitEvent(ctx.stream, ctx.ev[4 * (c - 2) + 3], 0));
-        TB_CK(cudaEventRecord(e[0], ctx.stream));
         // The chunk's striped pairs come first; alone they take `stream`, else a stream beside the fill's.
         const uint32_t n_str_pairs = run.m > 0 && n_striped > chunk_at[c] ? std::min(n_striped, chunk_at[c + 1]) - chunk_at[c] : 0;
         const bool beside = n_str_pairs > 0 && n_str_pairs < p.n_pairs;
+        const uint32_t n_str = n_str_pairs * per_pair;
+        if (n_str > 0) TB_CK(cudaMemsetAsync(ctx.d_prog + 4, 0, sizeof(uint32_t) * n_str, ctx.stream));
+        TB_CK(cudaEventRecord(e[0], ctx.stream));
         cudaEvent_t e_str = ctx.ev[4 * n_chunks + 2 + c];
-        if (n_str_pairs > 0) {
+        if (n_str > 0) {
             const cudaStream_t st = beside ? ctx.stream_s : ctx.stream;
-            if (beside) TB_CK(cudaStreamWaitEvent(st, e[0], 0));
-            const uint32_t n_str = n_str_pairs * per_pair;
+            if (beside) {
+                // The stripes need all their blocks resident at once, so the fill, whose blocks would take
+                // the places first, waits until the stripes' stream has come as far.
+                TB_CK(cudaStreamWaitEvent(st, e[0], 0));
+                TB_CK(cudaEventRecord(e_str, st));
+                TB_CK(cudaStreamWaitEvent(ctx.stream, e_str, 0));
+            }
             TbParams ps = p;
             ps.n_pairs = n_str_pairs;
             TbStripes S{ctx.d_first, n_str, tb_stripe_smem_al(run.al), ctx.d_bnd, ctx.d_prog + 4, (int *)ctx.d_prog,
                         tb_spin_limit()};
-            TB_CK(cudaMemsetAsync(S.prog, 0, sizeof(uint32_t) * n_str, st));
             TB_CK(dispatch_stripes(run.mode, true, ps, S, st, ctx.device));
             if (beside) TB_CK(cudaEventRecord(e_str, st));
             ctx.launches += 2;
