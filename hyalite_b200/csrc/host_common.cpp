@@ -20,6 +20,7 @@ static thread_local int64_t g_detail[3] = {0, 0, 0};
 static std::atomic<int64_t> g_live_allocs{0};
 static std::atomic<int64_t> g_fail_countdown{-1};
 static std::atomic<uint32_t> g_wait_polls{WAIT_POLLS_DEFAULT};
+static std::atomic<int64_t> g_row_wait_polls{-1};  // -1: as g_wait_polls
 static std::atomic<uint64_t> g_wait_epoch{0};
 
 cudaError_t dev_malloc_bytes(void **p, size_t bytes) {
@@ -45,6 +46,10 @@ cudaError_t dev_free(void *p) {
 }
 
 uint32_t wait_polls() { return g_wait_polls.load(); }
+uint32_t row_wait_polls() {
+    const int64_t v = g_row_wait_polls.load();
+    return v < 0 ? wait_polls() : (uint32_t)v;
+}
 uint64_t wait_polls_epoch() { return g_wait_epoch.load(); }
 
 hy_status fail(hy_status st, int64_t d0, int64_t d1, int64_t d2) {
@@ -231,6 +236,11 @@ int64_t hy_debug_live_device_allocations(void) { return hy::g_live_allocs.load()
 
 void hy_debug_set_wait_polls(int64_t polls) {
     hy::g_wait_polls.store(polls < 0 ? hy::WAIT_POLLS_DEFAULT : (uint32_t)std::min<int64_t>(polls, UINT32_MAX));
+    hy::g_wait_epoch.fetch_add(1);
+}
+
+void hy_debug_set_row_wait_polls(int64_t polls) {
+    hy::g_row_wait_polls.store(polls < 0 ? -1 : std::min<int64_t>(polls, UINT32_MAX));
     hy::g_wait_epoch.fetch_add(1);
 }
 

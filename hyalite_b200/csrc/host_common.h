@@ -25,7 +25,9 @@ cudaError_t dev_free(void *p);
 // parameter). The default bounds a wait to seconds; a test may lower it to make waits run out.
 constexpr uint32_t WAIT_POLLS_DEFAULT = 1u << 24;
 uint32_t wait_polls();
-// Counts the changes of wait_polls(): work captured into a CUDA graph under an older value (the
+// The same for a band block's waits for its neighbour's rows (wait_polls() unless a test sets it).
+uint32_t row_wait_polls();
+// Counts the changes of these limits: work captured into a CUDA graph under an older value (the
 // limit is a kernel parameter, frozen at capture) is captured again.
 uint64_t wait_polls_epoch();
 

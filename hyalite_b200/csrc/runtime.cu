@@ -362,6 +362,7 @@ static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &
     p.best_key = key;
     p.err = sc->d_err;
     p.wait_polls = wait_polls();
+    p.row_polls = row_wait_polls();
     set_extents<A>(p, db, part, part.total_cols);
     HY_CK(launch_band<A>(db->mode, sh, p, item_ptr ? 1 : item_end - item_base, st));
     sc->launches += qp.n_passes > 0 ? 2 : 1;
@@ -651,6 +652,7 @@ static hy_status band_pair_enqueue(BandPairContext &c, const uint8_t *d_q, uint6
     p.best_key = nullptr;
     p.err = reinterpret_cast<int *>(const_cast<uint8_t *>(base) + 36);
     p.wait_polls = wait_polls();
+    p.row_polls = row_wait_polls();
     p.res_cols = tl;
     p.bnd_cols = tl;
     p.n_seqs = slot + 1;

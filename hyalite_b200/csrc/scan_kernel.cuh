@@ -85,6 +85,7 @@ struct ScanParams {
     // query end, target end} instead of to scores / qend / tend.
     int32_t *ends_out;
     uint32_t wait_polls;  // polls a wait for a profile copy makes before it gives up
+    uint32_t row_polls;   // polls a band block waits for its neighbour's rows, or for ring space there
     // Extents the bounds-checked build (HY_BOUNDS) verifies every item against before use.
     uint64_t res_cols;  // columns of the residue array
     uint64_t bnd_cols;  // columns the boundary region holds, from bnd_col0
@@ -1450,6 +1451,13 @@ __global__ void __launch_bounds__((scan_max_threads<A, G, R>()), (scan_min_block
 // BAND_K pairs there), which gives each ring block back once read; the blocks share no other step
 // (a cluster barrier a window took 2850 cycles of its 3400).
 //
+// A wait between blocks that gives up ends its side of that link: a block that did not get its row
+// arms and gives back no more ring blocks, one that got no space sends none from that ring block on
+// (it has sent whole ring blocks then). Both sweep on, on rows that no one uses, so that every block
+// comes to the next cluster barrier, and there all stop: the error word is set, no result is written,
+// and before the barrier that lets the blocks exit a block waits for the ring blocks that were sent
+// to it and that it has not read, so that no row lands in the shared memory of a block that is gone.
+//
 // What bounds it is one warp's step: a lone warp issues a chain of dependent instructions with
 // nothing beside it (one column of 4 rows a step with plain loads: 66 instructions, 250 cycles). So a
 // step has two columns whose chains are independent but for a row's lag, and as few other instructions
@@ -1734,6 +1742,21 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     const int n_blk = (pairs + BAND_K - 1) / BAND_K;
     uint32_t full_ph = 0, empty_ph = 0;  // per slot: parity of its next wait at the round's start
     auto blk_bytes = [&](int blk) { return 16u * (uint32_t)min(BAND_K, pairs - blk * BAND_K); };
+    // The ring block at which this warp gave up on the row above or on space for its own row.
+    constexpr int NEVER = INT32_MAX;
+    int recv_end = NEVER, send_end = NEVER;
+    bool gave = false;           // any warp of the block has
+    __shared__ uint32_t s_sent;  // ring blocks of the round that this block has sent
+    // The wait for the rows still on their way to this block (every block's sweep is over).
+    auto drain = [&]() {
+        if (threadIdx.x == 0 && recv_end != NEVER) {
+            const int sent = (int)ld_cluster_u32(&s_sent, crank - 1);
+            for (int blk = recv_end; blk < sent; ++blk)
+                mbar_wait_cluster(full + blk % BAND_SLOTS, ((full_ph >> (blk % BAND_SLOTS)) + (uint32_t)(blk / BAND_SLOTS)) & 1u,
+                                  1u << 24);
+        }
+        __syncwarp();
+    };
     const int rounds = (p.n_passes + WT - 1) / WT;
     for (int round = 0; round < rounds; ++round) {
         const int first = round * WT;
@@ -1749,10 +1772,14 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                 phase ^= 1u;
                 fail = __syncthreads_or(!ok);
             }
-            if (csize > 1 && threadIdx.x == 0 && crank > 0 && bcnt > 0 && w > 0)
+            if (csize > 1 && threadIdx.x == 0 && crank > 0 && bcnt > 0 && w > 0 && !gave)
                 for (int blk = 0; blk < min(BAND_SLOTS, n_blk); ++blk) mbar_expect(full + blk, blk_bytes(blk));
-            if (cluster_any(fail, &s_flag, csize)) {
+            if (cluster_any(fail || gave, &s_flag, csize)) {
                 if (threadIdx.x == 0 && fail) wait_gave_up(p.err, bar, 1u, phase ^ 1u);  // the round's copy
+                if (csize > 1) {
+                    drain();
+                    cluster_barrier();
+                }
                 return;
             }
         }
@@ -1764,13 +1791,10 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
         const bool from_block = warp == 0 && crank > 0;
         const bool to_block = warp == W - 1 && gw + 1 < cnt;
         const bool to_bnd = !last_pass && gw + 1 == cnt;  // the round's last row: for the next round
-        bool waits = true;                                // until a wait gives up
-        auto wait_cluster = [&](uint64_t *b, uint32_t parity) {
-            if (waits && !mbar_wait_cluster(b, parity & 1u, p.wait_polls)) {
-                waits = false;
-                atomicExch(p.err, ERR_WAIT);
-            }
-            waits = __all_sync(0xffffffffu, waits);
+        auto wait_cluster = [&](uint64_t *b, uint32_t parity) -> bool {
+            const bool ok = mbar_wait_cluster(b, parity & 1u, p.row_polls);
+            if (!ok) atomicExch(p.err, ERR_WAIT);
+            return __all_sync(0xffffffffu, ok);
         };
         const int32_t row0 = p.vrow0 + pass * RPP + lane * R;
         const uint8_t *prof = GPROF ? p.profile + (size_t)min(pass, p.n_passes - 1) * p.pass_bytes
@@ -1856,12 +1880,15 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                     // Block b - 1's last warp writes the row above: the ring block read a window ago
                     // goes back to it, and the next one must have arrived.
                     const int blk = s0 / BAND_K, old = blk - 1;
-                    if (old >= 0 && old + BAND_SLOTS < n_blk && lane == 0) {
-                        mbar_expect(full + old % BAND_SLOTS, blk_bytes(old + BAND_SLOTS));
-                        mbar_arrive_cluster(cluster_addr(empty + old % BAND_SLOTS, crank - 1));
+                    if (recv_end == NEVER) {
+                        if (old >= 0 && old + BAND_SLOTS < n_blk && lane == 0) {
+                            mbar_expect(full + old % BAND_SLOTS, blk_bytes(old + BAND_SLOTS));
+                            mbar_arrive_cluster(cluster_addr(empty + old % BAND_SLOTS, crank - 1));
+                        }
+                        if (blk < n_blk &&
+                            !wait_cluster(full + blk % BAND_SLOTS, (full_ph >> (blk % BAND_SLOTS)) + (uint32_t)(blk / BAND_SLOTS)))
+                            recv_end = blk;
                     }
-                    if (blk < n_blk)
-                        wait_cluster(full + blk % BAND_SLOTS, (full_ph >> (blk % BAND_SLOTS)) + (uint32_t)(blk / BAND_SLOTS));
                 } else if (warp == 0 && lane < BAND_K) {
                     // The row above of the window's pairs: the top border, or the boundary row that
                     // the round before wrote.
@@ -1922,10 +1949,11 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                         // Pairs s0 - 31 .. s0 - 16, the last one the first of its ring block, whose
                         // earlier pairs the next block must have read.
                         const int blk = s0 / BAND_K - 1;
-                        if (blk >= BAND_SLOTS && blk < n_blk)
-                            wait_cluster(empty + blk % BAND_SLOTS,
-                                         (empty_ph >> (blk % BAND_SLOTS)) + (uint32_t)(blk / BAND_SLOTS - 1));
-                        if (has)
+                        if (send_end == NEVER && blk >= BAND_SLOTS && blk < n_blk &&
+                            !wait_cluster(empty + blk % BAND_SLOTS,
+                                          (empty_ph >> (blk % BAND_SLOTS)) + (uint32_t)(blk / BAND_SLOTS - 1)))
+                            send_end = blk;
+                        if (has && c / BAND_K < send_end)
                             st_async_v4(cluster_addr(in - (size_t)warp * BAND_RING + c % BAND_RING, crank + 1), out[c % BAND_RING],
                                         cluster_addr(full + (c / BAND_K) % BAND_SLOTS, crank + 1));
                     }
@@ -1933,13 +1961,15 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
             }
             __syncthreads();
         }
+        if (to_block && lane == 0) s_sent = (uint32_t)min(send_end, n_blk);
+        if (mine) band_end<A, R, MODE>(sw, row0, p.go, copy, cand);
+        gave = __syncthreads_or(recv_end != NEVER || send_end != NEVER);  // the slices and rings may be refilled
+        if (gave) continue;  // (the phases stay those of the round that gave up)
         for (int k2 = 0; k2 < BAND_SLOTS; ++k2) {
             const int uses = n_blk > k2 ? (n_blk - k2 + BAND_SLOTS - 1) / BAND_SLOTS : 0;
             full_ph ^= (uint32_t)(uses & 1) << k2;
             empty_ph ^= (uint32_t)(max(uses - 1, 0) & 1) << k2;
         }
-        if (mine) band_end<A, R, MODE>(sw, row0, p.go, copy, cand);
-        __syncthreads();  // the slices and rings may be refilled for the next round
     }
     // Reduce every lane's candidates: inside each warp, then across warps in shared memory.
     __shared__ Cand s_cand[32][2];
@@ -1960,7 +1990,9 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
         cluster_barrier();  // every block's candidates are in its shared memory
     else
         __syncthreads();
-    if (threadIdx.x == 0 && crank == 0) {
+    if (csize > 1) drain();
+    // (A block of the cluster that gave up has set the error word before the barrier.)
+    if (threadIdx.x == 0 && crank == 0 && (csize == 1 || *(volatile int *)p.err == 0)) {
         for (int h = 0; h < A::NH; ++h) {
             const uint32_t idx = meta.idx[h];
             if (idx == NO_INDEX) continue;
