@@ -325,6 +325,22 @@ extern "C" void hy_debug_band_shape(uint32_t pass_bytes, int32_t n_passes, uint6
     out[3] = (n_passes + sh.warps * sh.blocks - 1) / (sh.warps * sh.blocks);
 }
 
+extern "C" hy_status hy_debug_band_plan(int arith, uint64_t al, uint64_t qlen, uint64_t smem_limit, uint64_t out[6]) {
+    if (!out || arith < 0 || arith > 2 || al > 255 || qlen >= (1u << 30)) return hy::fail(HY_ERR_INVALID_ARGUMENT);
+    hy::QueryPlan qp;
+    const hy::BandShape sh = arith == 0   ? hy::band_plan<hy::Pair16>(qlen, al, smem_limit, qp)
+                             : arith == 1 ? hy::band_plan<hy::PairTab16>(qlen, al, smem_limit, qp)
+                                          : hy::band_plan<hy::Single32>(qlen, al, smem_limit, qp);
+    const uint64_t warps = (uint64_t)sh.warps * sh.blocks;
+    out[0] = (uint64_t)sh.rows;
+    out[1] = sh.gprof ? 1 : 0;
+    out[2] = (uint64_t)sh.warps;
+    out[3] = (uint64_t)sh.blocks;
+    out[4] = ((uint64_t)qp.n_passes + warps - 1) / warps;
+    out[5] = sh.smem;
+    return hy::fail(HY_OK);
+}
+
 namespace hy {
 
 // Scores and end positions of the single item *item_ptr, or of the items [item_base, item_end) (a

@@ -1498,10 +1498,13 @@ constexpr int BAND_SLOTS = BAND_RING / BAND_K;
 constexpr int BAND_BARS = 1 + 2 * BAND_SLOTS;
 
 // Shared memory of a band block of `warps` warps with pass slices of `slice` bytes (0: in global
-// memory): the slices, the rings, the rest of the warps' bytes, the mbarrier.
+// memory): the slices, the rings (at the end the warps' candidates in their place), the rest of the
+// warps' bytes, the mbarriers, two words. All of it dynamic, so that the host's sum is what a block takes.
+constexpr size_t BAND_TAIL_BYTES = BAND_BARS * 8 + 8;
 __host__ __device__ inline size_t band_smem_bytes(size_t warps, size_t slice, int rows) {
-    return warps * (slice + band_warp_bytes(rows)) + BAND_RING_BYTES + BAND_BARS * 8;
+    return warps * (slice + band_warp_bytes(rows)) + BAND_RING_BYTES + BAND_TAIL_BYTES;
 }
+static_assert(BAND_RING_BYTES >= 2 * sizeof(Cand), "a warp's candidates must fit in its ring");
 
 // A band lane's state: a Sweep's, with the last row of both columns.
 template <class A, int R>
@@ -1708,7 +1711,6 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     const int crank = cluster_rank(), csize = cluster_size();
     const int WT = W * csize;          // warps of the cluster
     const int gw = crank * W + warp;   // this warp's index in the cluster
-    __shared__ uint32_t s_flag;
     const ItemMeta meta = p.meta[item];
 #ifdef HY_BOUNDS
     // Every warp checks the item (the same answer in all of them), so all skip it together.
@@ -1728,6 +1730,10 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     uint4 *out = in + BAND_RING;
     uint8_t *own = rings + (size_t)(W + 1) * BAND_RING_BYTES + (size_t)warp * (band_warp_bytes(R) - BAND_RING_BYTES);
     W2 *strip = reinterpret_cast<W2 *>(own);
+    uint32_t *words = reinterpret_cast<uint32_t *>(rings + (size_t)(W + 1) * BAND_RING_BYTES +
+                                                   (size_t)W * (band_warp_bytes(R) - BAND_RING_BYTES) + BAND_BARS * 8);
+    uint32_t &s_flag = words[0];
+    uint32_t &s_sent = words[1];  // ring blocks of the round that this block has sent
     uint4 *copy = reinterpret_cast<uint4 *>(own + BAND_STRIP_BYTES) + lane;
     SweepConst<A> k;
     k.negge = A::splat(-(int64_t)p.ge);
@@ -1746,7 +1752,6 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     constexpr int NEVER = INT32_MAX;
     int recv_end = NEVER, send_end = NEVER;
     bool gave = false;           // any warp of the block has
-    __shared__ uint32_t s_sent;  // ring blocks of the round that this block has sent
     // The wait for the rows still on their way to this block (every block's sweep is over).
     auto drain = [&]() {
         if (threadIdx.x == 0 && recv_end != NEVER) {
@@ -1816,7 +1821,7 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
         W2 c_prev = 0, c_cur = 0, c_next = 0;  // (0: a valid letter)
         V pa[2][R], pb[2][R];  // profile words of the coming step
         uint32_t code = 0;     // residue codes of the step after it
-        auto words = [&](const uint32_t cc, V (&a)[2][R], V (&b)[2][R]) {
+        auto prof_words = [&](const uint32_t cc, V (&a)[2][R], V (&b)[2][R]) {
             band_words<A, R>(prof, prof_hi, cc & CODE_MASK, lane, a[0], b[0]);
             band_words<A, R>(prof, prof_hi, cc >> CODE_BITS, lane, a[1], b[1]);
         };
@@ -1826,7 +1831,7 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
             strip[lane] = 0;
             strip[G + lane] = c_cur;
             __syncwarp();
-            words(strip[G - lane], pa, pb);
+            prof_words(strip[G - lane], pa, pb);
             code = strip[G + 1 - lane];
         }
         // Step s = s0 + i of the window at s0: `up` the row above at lane 0's pair, `cp` the strip at
@@ -1844,7 +1849,7 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                 upF1 = (V)up.w;
             }
             V na[2][R], nb[2][R];
-            words(code, na, nb);
+            prof_words(code, na, nb);
             code = cp[i + 2];
             constexpr bool edge = decltype(EDGE)::value;
             const int c = s0 + i - lane;
@@ -1972,8 +1977,8 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
         }
     }
     // Reduce every lane's candidates: inside each warp, then across warps in shared memory.
-    __shared__ Cand s_cand[32][2];
-    __syncthreads();  // a previous item's reduction may still be reading s_cand
+    Cand(*s_cand)[2] = reinterpret_cast<Cand(*)[2]>(rings);  // (the last round's rings have been read)
+    __syncthreads();
 #pragma unroll
     for (int h = 0; h < A::NH; ++h) {
 #pragma unroll
@@ -1991,8 +1996,9 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     else
         __syncthreads();
     if (csize > 1) drain();
-    // (A block of the cluster that gave up has set the error word before the barrier.)
-    if (threadIdx.x == 0 && crank == 0 && (csize == 1 || *(volatile int *)p.err == 0)) {
+    if (threadIdx.x == 0 && crank == 0) {
+        // A block of the cluster that gave up has set the error word before the barrier.
+        const int err = csize > 1 ? *(volatile int *)p.err : 0;
         for (int h = 0; h < A::NH; ++h) {
             const uint32_t idx = meta.idx[h];
             if (idx == NO_INDEX) continue;
@@ -2007,6 +2013,7 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
                     }
                     if (better(o, c)) c = o;
                 }
+            if (err) continue;
             if (p.ends_out) {
                 if (idx == ~(uint32_t)(*p.best_key & 0xffffffffu)) {
                     p.ends_out[0] = c.s;
@@ -2038,7 +2045,7 @@ __global__ void __launch_bounds__(32 * band_max_warps<R>(), 1) band_kernel(const
     const uint32_t item = p.item_ptr ? *p.item_ptr : p.item_base + blockIdx.x / (uint32_t)cluster_size();
     if (item == NO_INDEX || item >= p.n_items) return;  // the same for every thread of the cluster
     const int W = blockDim.x / 32;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + band_smem_bytes(W, GPROF ? 0 : p.pass_bytes, R)) - BAND_BARS;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + band_smem_bytes(W, GPROF ? 0 : p.pass_bytes, R) - BAND_TAIL_BYTES);
     if (threadIdx.x == 0) {
         for (int i = 0; i < BAND_BARS; ++i) mbar_init(bar + i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
