@@ -158,6 +158,16 @@ struct PairsContext {
         for (cudaEvent_t e : {ev_fork, ev_side, ev_long})
             if (e) cudaEventDestroy(e);
     }
+    // Whether no work is left on any stream, and the wait for it.
+    bool idle() const {
+        for (cudaStream_t s : {stream, copy_stream, d2h_stream, side_stream, long_stream})
+            if (s && cudaStreamQuery(s) != cudaSuccess) return false;
+        return true;
+    }
+    void drain() const {
+        for (cudaStream_t s : {copy_stream, side_stream, long_stream, stream, d2h_stream})
+            if (s) cudaStreamSynchronize(s);
+    }
     cudaError_t get_pinned(int slot, size_t bytes, void **out) {
         bytes = std::max<size_t>(bytes, 16);
         if (pinned[slot].n < bytes) {
@@ -955,6 +965,15 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
                 HY_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
             for (cudaEvent_t &e : ctx.slot_ev) HY_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         }
+        // A call that fails part-way leaves no work behind: the next call's copies would overwrite, on
+        // another stream, the queries, items and staging slots that its kernels still read.
+        struct DrainOnReturn {
+            PairsContext &ctx;
+            bool done = false;
+            ~DrainOnReturn() {
+                if (!done) ctx.drain();
+            }
+        } drain_on_return{ctx};
         const uint64_t L = n_len;
         const std::vector<uint64_t> bounds = plan_pair_chunks(q_off, t_off, L);
         const uint64_t n_chunks = bounds.size() - 1;
@@ -1291,6 +1310,7 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             }
         }
         HY_CK(cudaStreamSynchronize(ctx.stream));
+        drain_on_return.done = true;
         if (h_cm && !cm_direct)
             for (uint32_t k : run_long)
                 memcpy(pc.colmax + (t_off[k] - t_off[0]), h_cm + (t_off[k] - t_off[0]),
@@ -1408,6 +1428,9 @@ extern "C" hy_status hy_align_pairs_phases(double *ms, uint32_t n) {
     for (uint32_t i = 0; i < n && i < 7; ++i) ms[i] = g_ctx.phase_ms[i];
     return fail(HY_OK);
 }
+
+// Whether the calling thread's last align_pairs call has left no work on the device.
+extern "C" int hy_debug_pairs_idle(void) { return g_ctx.idle() ? 1 : 0; }
 
 // The chunk boundaries hy_align_pairs would use for these offsets (introspection for tests):
 // writes up to `cap` boundaries and returns the number of chunks.
