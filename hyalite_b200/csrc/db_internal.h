@@ -20,7 +20,7 @@ constexpr int MAIN_G32 = 32;
 constexpr int MAIN_R32 = 16;
 constexpr int WIN_G = 32;
 constexpr int WIN_R = 8;
-constexpr int BAND_FEW_ROWS = 4;  // rows per lane of a band whose passes then still fit one round
+constexpr int BAND_FEW_ROWS = 4;  // rows per lane of a scan's or a long pair's band
 // The batched form's pairs longer than LONG_W columns run one full warp each (LONG_G lanes of
 // LONG_R rows) in a class of their own, whose boundary regions the bulk classes then need not
 // size for. Plain scans keep every pair in the bulk kernel (measured: the same time as a separate

@@ -239,16 +239,18 @@ static cudaError_t launch_band_mode(const ScanParams &p, int warps, int blocks, 
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-// Launch shape of the band kernel for a query plan: one pass slice per warp in shared memory (a
-// slice too large for that runs from the profile in global memory, 32 warps on one block); more
-// passes than one block's slices hold take a cluster of blocks, so that the passes run in as few
-// rounds as possible.
+// Launch shape of the band kernel.
 struct BandShape {
     bool gprof;
     int warps, blocks;
     size_t smem;
     int rows;  // rows per lane
+    int rounds;
 };
+// A shape of 8 rows per lane for a query plan: one pass slice per warp in shared memory (a slice too
+// large for that: in global memory, on one block), up to 32 warps a block; more passes than one block's
+// slices hold take a cluster of blocks, so that the passes run in as few rounds as possible. What fits
+// one round of it decides which lone pairs take the band kernel (band_long_pair_fits).
 static BandShape band_shape(const QueryPlan &qp, size_t smem_limit) {
     BandShape sh;
     const size_t budget = std::min<size_t>(BAND_SMEM_BUDGET, smem_limit - band_smem_bytes(1, 0, WIN_R));
@@ -267,32 +269,60 @@ static BandShape band_shape(const QueryPlan &qp, size_t smem_limit) {
     sh.warps = warps;
     sh.blocks = blocks;
     sh.smem = band_smem_bytes(warps, sh.gprof ? 0 : qp.pass_bytes, WIN_R);
+    sh.rounds = std::max(1, (qp.n_passes + blocks * warps - 1) / (blocks * warps));
     return sh;
 }
 
-// The shape a band of lane arithmetic A runs a query of length qlen in, and its plan: 4 rows per lane
-// on blocks of 4 warps, so that a warp has its scheduler to itself, on up to 8 blocks of a cluster,
-// and more warps a block beyond that, while all passes fit one round of at most 16 warps a block;
-// else 8 rows per lane. (2000 x 2000 / 5000 x 5000 int32 pair: 0.231 / 0.674 ms; 2 warps a block 0.229
-// / 0.674, and 0.27 against 0.22 for 3 passes; 8 warps 0.268 / 0.712; 8 rows per lane 0.61 / 1.65.)
+// `passes` passes in as few rounds as `most` warps a block and a cluster of 8 allow, a round's passes 4
+// warps a block while 8 blocks hold them, so that a warp has its scheduler to itself.
+static BandShape band_rounds(const QueryPlan &qp, int rows, int most) {
+    const int passes = std::max(1, qp.n_passes);
+    const int rounds = (passes + BAND_CLUSTER_MAX * most - 1) / (BAND_CLUSTER_MAX * most);
+    const int per = (passes + rounds - 1) / rounds;
+    const int blocks = std::max((per + most - 1) / most, std::min(BAND_CLUSTER_MAX, (per + 3) / 4));
+    const int warps = (per + blocks - 1) / blocks;
+    return {false, warps, blocks, band_smem_bytes(warps, qp.pass_bytes, rows), rows, rounds};
+}
+
+// Warps of `rows` rows per lane whose slices fit in a block's shared memory, up to BAND_WARPS.
+static int band_warps_fit(const QueryPlan &qp, int rows, size_t smem_limit) {
+    const size_t fixed = band_smem_bytes(0, 0, rows), each = qp.pass_bytes + band_warp_bytes(rows);
+    return (int)std::min<size_t>(BAND_WARPS, smem_limit > fixed ? (smem_limit - fixed) / each : 0);
+}
+
+// The shape a band of lane arithmetic A runs a query of length qlen in, and its plan: 4 rows per lane.
+// (2000 x 2000 / 5000 x 5000 int32 pair: 0.231 / 0.674 ms; 2 warps a block 0.229 / 0.674, and 0.27
+// against 0.22 for 3 passes; 8 warps 0.268 / 0.712; 8 rows per lane 0.61 / 1.65.) Where those take more
+// rounds than 8 rows per lane would, the modes with the long row chain run 8 (16,400 x 3000, two rounds
+// against one: 1.65 and 1.28 ms in global mode; local mode, whose chain is short, 1.86 and 2.02). A slice
+// that does not fit a block's shared memory is read from global memory, by 8 rows per lane on one block.
 template <class A>
-static BandShape band_plan(uint64_t qlen, uint64_t al, size_t smem_limit, QueryPlan &qp) {
+static BandShape band_plan(uint64_t qlen, uint64_t al, size_t smem_limit, int mode, QueryPlan &qp) {
     qp = plan_for<A>(qlen, WIN_G * BAND_FEW_ROWS, al);
-    const int blocks = std::max(1, std::min(BAND_CLUSTER_MAX, (qp.n_passes + 3) / 4));
-    const int warps = std::max(1, (qp.n_passes + blocks - 1) / blocks);
-    const size_t smem = band_smem_bytes(warps, qp.pass_bytes, BAND_FEW_ROWS);
-    if (warps <= band_max_warps<BAND_FEW_ROWS>() && smem <= smem_limit) return {false, warps, blocks, smem, BAND_FEW_ROWS};
-    qp = plan_for<A>(qlen, WIN_G * WIN_R, al);
-    return band_shape(qp, smem_limit);
+    const int most = band_warps_fit(qp, BAND_FEW_ROWS, smem_limit);
+    const QueryPlan qp8 = plan_for<A>(qlen, WIN_G * WIN_R, al);
+    if (most > 0) {
+        const BandShape sh = band_rounds(qp, BAND_FEW_ROWS, most);
+        const int most8 = mode == MODE_SW ? 0 : band_warps_fit(qp8, WIN_R, smem_limit);
+        if (sh.rounds == 1 || most8 == 0) return sh;
+        const BandShape sh8 = band_rounds(qp8, WIN_R, most8);
+        if (sh8.rounds >= sh.rounds) return sh;
+        qp = qp8;
+        return sh8;
+    }
+    qp = qp8;
+    const int warps = std::max(1, std::min(BAND_WARPS, qp.n_passes));
+    return {true, warps, 1, band_smem_bytes(warps, 0, WIN_R), WIN_R, std::max(1, (qp.n_passes + warps - 1) / warps)};
 }
 
 template <class A>
 static cudaError_t launch_band(int mode, const BandShape &sh, const ScanParams &p, uint32_t items, cudaStream_t st) {
 #define HY_BAND_CASE(M)                                                                                     \
     case M:                                                                                                 \
-        return sh.gprof             ? launch_band_mode<A, WIN_R, M, true>(p, sh.warps, 1, sh.smem, items, st)      \
-               : sh.rows == WIN_R   ? launch_band_mode<A, WIN_R, M, false>(p, sh.warps, sh.blocks, sh.smem, items, st) \
-                                    : launch_band_mode<A, BAND_FEW_ROWS, M, false>(p, sh.warps, sh.blocks, sh.smem, items, st);
+        if (sh.gprof) return launch_band_mode<A, WIN_R, M, true>(p, sh.warps, 1, sh.smem, items, st); \
+        if constexpr (M != MODE_SW)                                                                         \
+            if (sh.rows == WIN_R) return launch_band_mode<A, WIN_R, M, false>(p, sh.warps, sh.blocks, sh.smem, items, st); \
+        return launch_band_mode<A, BAND_FEW_ROWS, M, false>(p, sh.warps, sh.blocks, sh.smem, items, st);
     switch (mode) {
         HY_BAND_CASE(MODE_SW)
         HY_BAND_CASE(MODE_NW)
@@ -325,18 +355,17 @@ extern "C" void hy_debug_band_shape(uint32_t pass_bytes, int32_t n_passes, uint6
     out[3] = (n_passes + sh.warps * sh.blocks - 1) / (sh.warps * sh.blocks);
 }
 
-extern "C" hy_status hy_debug_band_plan(int arith, uint64_t al, uint64_t qlen, uint64_t smem_limit, uint64_t out[6]) {
-    if (!out || arith < 0 || arith > 2 || al > 255 || qlen >= (1u << 30)) return hy::fail(HY_ERR_INVALID_ARGUMENT);
+extern "C" hy_status hy_debug_band_plan(int arith, int mode, uint64_t al, uint64_t qlen, uint64_t smem_limit, uint64_t out[6]) {
+    if (!out || arith < 0 || arith > 2 || mode < 0 || mode > 4 || al > 255 || qlen >= (1u << 30)) return hy::fail(HY_ERR_INVALID_ARGUMENT);
     hy::QueryPlan qp;
-    const hy::BandShape sh = arith == 0   ? hy::band_plan<hy::Pair16>(qlen, al, smem_limit, qp)
-                             : arith == 1 ? hy::band_plan<hy::PairTab16>(qlen, al, smem_limit, qp)
-                                          : hy::band_plan<hy::Single32>(qlen, al, smem_limit, qp);
-    const uint64_t warps = (uint64_t)sh.warps * sh.blocks;
+    const hy::BandShape sh = arith == 0   ? hy::band_plan<hy::Pair16>(qlen, al, smem_limit, mode, qp)
+                             : arith == 1 ? hy::band_plan<hy::PairTab16>(qlen, al, smem_limit, mode, qp)
+                                          : hy::band_plan<hy::Single32>(qlen, al, smem_limit, mode, qp);
     out[0] = (uint64_t)sh.rows;
     out[1] = sh.gprof ? 1 : 0;
     out[2] = (uint64_t)sh.warps;
     out[3] = (uint64_t)sh.blocks;
-    out[4] = ((uint64_t)qp.n_passes + warps - 1) / warps;
+    out[4] = (uint64_t)sh.rounds;
     out[5] = sh.smem;
     return hy::fail(HY_OK);
 }
@@ -351,7 +380,7 @@ static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &
                               int32_t *scores, uint8_t *prof, void *bnd, const uint32_t *item_ptr, cudaStream_t st) {
     const bool i16 = A::NH == 2;
     QueryPlan qp;
-    const BandShape sh = band_plan<A>(qlen, db->al, db->smem_limit, qp);
+    const BandShape sh = band_plan<A>(qlen, db->al, db->smem_limit, db->mode, qp);
     const int32_t lim = i16 ? lim16(db) : LIM32;
     if (sh.rows == WIN_R)
         HY_CK((launch_profile<A, WIN_G, WIN_R>(db, d_query, qlen, qp, lim, prof, st)));
@@ -439,8 +468,9 @@ static ScanForms forms_for(const hy_db *db, const QuerySplit &split, uint64_t ql
     ScanForms f = scan_forms(db, split, qlen, ends, bulk_rows_for<P>(db, qlen, ends), g, r,
                              r == 16 ? wide_threads<P>(db, qlen) : BLOCK);
     QueryPlan bp;
-    if (band_plan<P>(qlen, db->al, db->smem_limit, bp).rows != BAND_FEW_ROWS) f.band_end = split.k0;
-    if (band_plan<Single32>(qlen, db->al, db->smem_limit, bp).rows != BAND_FEW_ROWS) f.band32 = false;
+    auto one_round = [](const BandShape &sh) { return sh.rows == BAND_FEW_ROWS && sh.rounds == 1; };
+    if (!one_round(band_plan<P>(qlen, db->al, db->smem_limit, db->mode, bp))) f.band_end = split.k0;
+    if (!one_round(band_plan<Single32>(qlen, db->al, db->smem_limit, db->mode, bp))) f.band32 = false;
     const QueryPlan wp = plan_for<P>(qlen, g * r, db->al);
     if (scan_slices(wp.n_passes) * (size_t)wp.pass_bytes + scan_extra_smem(2, r, db->mode, ends, BLOCK) > db->smem_limit)
         f.wide_end = f.band_end;
@@ -617,7 +647,7 @@ static hy_status band_pair_enqueue(BandPairContext &c, const uint8_t *d_q, uint6
                                    cudaStream_t st, uint32_t slot, int32_t *d_scores, int32_t *d_qend,
                                    int32_t *d_tend) {
     QueryPlan qp;
-    const BandShape sh = band_plan<Single32>(m, al, c.smem_limit, qp);
+    const BandShape sh = band_plan<Single32>(m, al, c.smem_limit, mode, qp);
     HY_CK(grow_dev(c.prof, c.c_prof, std::max<size_t>(16, (size_t)qp.pass_bytes * qp.n_passes)));
     HY_CK(grow_dev(c.bnd, c.c_bnd, sizeof(int32_t) * (2 * tl + 16)));
     // The item (the target as one int32 column run, the pair's slot as its index), its index and

@@ -2031,15 +2031,12 @@ __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t it
     if (csize > 1) cluster_barrier();  // block 0 has read every block's candidates
 }
 
-// Warps of a band block at most: 32 where a block holds as many slices as fit (8 rows per lane),
-// 16 (128 registers a thread, no spills) for the form with fewer rows per lane.
-template <int R>
-constexpr int band_max_warps() {
-    return R < 8 ? 16 : 32;
-}
+// Warps of a band block at most: 128 registers a thread. (The sweep of two columns needs 110 to 124 with
+// 4 rows per lane; at 64, for 32 warps, 8 rows spilled 0.4 to 2 KB a thread and took twice as long.)
+constexpr int BAND_WARPS = 16;
 
 template <class A, int R, int MODE, bool GPROF = false>
-__global__ void __launch_bounds__(32 * band_max_warps<R>(), 1) band_kernel(const ScanParams p) {
+__global__ void __launch_bounds__(32 * BAND_WARPS, 1) band_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     // The item *item_ptr, or an item a cluster.
     const uint32_t item = p.item_ptr ? *p.item_ptr : p.item_base + blockIdx.x / (uint32_t)cluster_size();

@@ -258,16 +258,17 @@ int hy_debug_pairs_idle(void);
 /* Test hook: the forms one scan of a query of qlen residues runs its items in: {int32 items, whether
  * those take the band kernel, then int16x2 pairs on the band kernel, a warp each, in the bulk kernel}. */
 void hy_debug_scan_forms(const hy_db *db, uint64_t qlen, int ends, uint32_t out[5]);
-/* The launch shape of the end-recovery band kernel (a scan's winner, a long pair) for a query of
- * n_passes pass slices of pass_bytes each, with smem_limit bytes of shared memory a block: out =
- * {slices read from global memory (1) or shared memory (0), warps a block, blocks of the cluster,
- * rounds}. One slice per warp; more passes than one block holds take a cluster of up to 8 blocks. */
+/* A launch shape of 8 rows per lane and up to 32 warps a block for a query of n_passes pass slices of
+ * pass_bytes each, with smem_limit bytes of shared memory a block: out = {slices read from global memory
+ * (1) or shared memory (0), warps a block, blocks of the cluster, rounds}. One slice per warp; more passes
+ * than one block holds take a cluster of up to 8 blocks. A lone long pair that takes one round of it runs
+ * on the band kernel (in hy_debug_band_plan's shape), one that takes more on the stripe kernel. */
 void hy_debug_band_shape(uint32_t pass_bytes, int32_t n_passes, uint64_t smem_limit, int32_t out[4]);
-/* The band kernel's whole launch shape for a query of qlen residues over an alphabet of `al`: lane
- * arithmetic 0 int16x2 pairs, 1 pairs of the Precomputed layout, 2 int32; out = {rows per lane, slices
- * read from global memory (1) or shared memory (0), warps a block, blocks of the cluster, rounds, bytes
- * of shared memory a block}. hy_debug_band_shape is its fallback where 4 rows per lane do not fit. */
-hy_status hy_debug_band_plan(int arith, uint64_t al, uint64_t qlen, uint64_t smem_limit, uint64_t out[6]);
+/* The band kernel's launch shape for a query of qlen residues over an alphabet of `al`: lane arithmetic
+ * 0 int16x2 pairs, 1 pairs of the Precomputed layout, 2 int32; out = {rows per lane, slices read from
+ * global memory (1) or shared memory (0), warps a block, blocks of the cluster, rounds, bytes of shared
+ * memory a block}. */
+hy_status hy_debug_band_plan(int arith, int mode, uint64_t al, uint64_t qlen, uint64_t smem_limit, uint64_t out[6]);
 
 /* ---- batched scan (no reference counterpart: the reference scans one query per call) ---------- */
 
