@@ -44,6 +44,8 @@ inline int bulk_rows(uint64_t qlen, bool local_ends = false) {
 constexpr int BULK_MAX_RPP = 8 * 32;
 constexpr int WIDE_MAX_RPP = 32 * 16;
 constexpr size_t BAND_SMEM_BUDGET = 200 * 1024;
+// Shared memory of an SM (B200), and what each resident block reserves of it.
+constexpr size_t SM_SMEM = 228 * 1024, BLOCK_SMEM_RESERVE = 1024;
 // Blocks of one band-kernel cluster at most (the portable cluster size).
 constexpr int BAND_CLUSTER_MAX = 8;
 
@@ -228,8 +230,8 @@ constexpr double COST_SCHEDULERS = 148 * 4, COST_BUSY = 1.46, COST_ALONE = 2.2, 
 inline double band_chain(uint64_t qlen, double w) {
     return (w / 2 + 51 + 48 * (double)((qlen - 1) / 128)) * 100;
 }
-// A band's warps hold their places for the whole chain, two or three to a scheduler (shared memory),
-// busy or not: 134 to 152 busy-rate instructions a step measured (72 items of 40 passes, 1093 of 3).
+// A band's warps hold their places for the whole chain, busy or not: 134 to 152 busy-rate instructions a
+// step measured (72 items of 40 passes, 1093 of 3).
 inline double band_work(uint64_t qlen, double w) { return (double)((qlen + 127) / 128) * band_chain(qlen, w) * 1.5; }
 
 // Estimated cycles of `work` warp-instructions: the chip at its busy rate, then what is left of the
@@ -248,8 +250,9 @@ struct ScanLoad {
     }
 };
 
+// hold, hold32: what bands of pairs and of int32 items take beyond band_work, at least 1.
 inline ScanForms scan_forms(const hy_db *db, const QuerySplit &split, uint64_t qlen, bool ends, int bulk_r,
-                            int wide_g, int wide_r, int wide_threads) {
+                            int wide_g, int wide_r, int wide_threads, double hold, double hold32) {
     ScanForms f;
     f.wide_g = wide_g;
     f.wide_r = wide_r;
@@ -322,6 +325,21 @@ inline ScanForms scan_forms(const hy_db *db, const QuerySplit &split, uint64_t q
         const double t = time(f.band_end, f.wide_end, !f.band32);
         if (t < best) f.band32 = !f.band32;
     }
+    // Bands whose blocks leave a scheduler few warps stay only where they are still the sooner form of the
+    // items they took, by themselves.
+    auto alone = [](double count, double work, double chain) {
+        return std::max(count * work / COST_SCHEDULERS * COST_BUSY, chain);
+    };
+    if (f.band32 && hold32 > 1.0 &&
+        alone(split.n_i32, band_work(qlen, mean32) * hold32, band_chain(qlen, w32) * 2.35) >
+            alone(split.n_i32, cost.chain(qlen, 32, MAIN_R32, mean32), cost.chain(qlen, 32, MAIN_R32, w32) * 2.35))
+        f.band32 = false;
+    const double bands = f.band_end - k0, mean16 = mean(k0, f.band_end);
+    if (bands > 0 && hold > 1.0 &&
+        alone(bands, band_work(qlen, mean16) * hold, band_chain(qlen, width(k0)) * 2.35) >
+            alone(bands, cost.chain(qlen, f.wide_g, f.wide_r, mean16) * f.wide_g / 32,
+                  cost.chain(qlen, f.wide_g, f.wide_r, width(k0)) * (wide_threads > BLOCK ? 3.7 : 3.0)))
+        f.band_end = k0;
     return f;
 }
 

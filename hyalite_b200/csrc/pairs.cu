@@ -393,9 +393,6 @@ static cudaError_t launch_pairs_rows(int rows, int mode, bool ends, const PairPa
     }
 }
 
-// Shared memory of an SM (B200), and what each resident block reserves of it.
-constexpr size_t SM_SMEM = 228 * 1024, BLOCK_SMEM_RESERVE = 1024;
-
 // Groups per block of the pair kernel for group profiles of gb bytes: up to 256 threads, whole
 // warps, within PAIR_SMEM_LIMIT; 0 when not one warp of groups fits (the global-profile form).
 static int pair_groups_per_block(size_t gb, int G) {

@@ -458,6 +458,20 @@ static int bulk_rows_for(const hy_db *db, uint64_t qlen, bool ends) {
                : rows;
 }
 
+// What a band's work takes of the chip beyond the estimate for schedulers with enough warps, by how many
+// warps of this shape an SM's shared memory and registers leave a scheduler. int32 items that all run on the
+// band kernel, measured against that estimate: 0.5 to 0.9 with 3 or 4 warps to a scheduler; on clusters 0.9
+// to 2.3 with 2, 1.5 to 3.3 with 1, 1.7 to 7 below; on one block 0.8 with 1.5, 2.5 with a half. (50 letters,
+// 1,439 residues, 1,270 int32 items: 5.7 ms on the band kernel, which the estimate took for 2.4, and 2.6 a
+// warp each; 250 letters, 777 residues, 72 of 150 columns: 0.33 and 0.17. Pairs on one block, 150 letters,
+// 39 residues, 1,627 targets: 0.16 and 0.07; on clusters the pairs' estimate holds as it is: 50 letters,
+// 2,068 residues, 481 targets 1.4 ms with bands and 2.8 without.)
+static double band_hold(const BandShape &sh, bool i32) {
+    const size_t by_smem = SM_SMEM / (sh.smem + BLOCK_SMEM_RESERVE), by_regs = 65536 / (128 * 32 * (size_t)sh.warps);
+    const double warps = (double)(std::min(by_smem, by_regs) * sh.warps) / 4;
+    return std::max(1.0, (sh.blocks == 1 ? 1.25 : i32 ? 3.0 : 0.0) / warps);
+}
+
 // The forms a scan's items run in. An alphabet whose wide slices do not fit in shared memory keeps
 // every pair in the bulk kernel, and one whose band slices do not, every item out of the band kernel.
 template <class P>
@@ -465,12 +479,18 @@ static ScanForms forms_for(const hy_db *db, const QuerySplit &split, uint64_t ql
     int g, r;
     wide_shape(qlen, &g, &r);
     if (r == 16 && wide_threads<P>(db, qlen) > BLOCK && db->mode == MODE_SW && ends) r = 8;  // no room for the copies
+    QueryPlan bp, bp32;
+    const BandShape band = band_plan<P>(qlen, db->al, db->smem_limit, db->mode, bp);
+    const BandShape band32 = band_plan<Single32>(qlen, db->al, db->smem_limit, db->mode, bp32);
     ScanForms f = scan_forms(db, split, qlen, ends, bulk_rows_for<P>(db, qlen, ends), g, r,
-                             r == 16 ? wide_threads<P>(db, qlen) : BLOCK);
-    QueryPlan bp;
-    auto one_round = [](const BandShape &sh) { return sh.rows == BAND_FEW_ROWS && sh.rounds == 1; };
-    if (!one_round(band_plan<P>(qlen, db->al, db->smem_limit, db->mode, bp))) f.band_end = split.k0;
-    if (!one_round(band_plan<Single32>(qlen, db->al, db->smem_limit, db->mode, bp))) f.band32 = false;
+                             r == 16 ? wide_threads<P>(db, qlen) : BLOCK, band_hold(band, false),
+                             band_hold(band32, true));
+    // (Bands of several rounds, or on more blocks than 4 warps each would need, are for winners alone.)
+    auto full_blocks = [](const BandShape &sh, const QueryPlan &bp) {
+        return sh.rows == BAND_FEW_ROWS && sh.rounds == 1 && sh.blocks <= std::max(1, std::min(BAND_CLUSTER_MAX, (bp.n_passes + 3) / 4));
+    };
+    if (!full_blocks(band, bp)) f.band_end = split.k0;
+    if (!full_blocks(band32, bp32)) f.band32 = false;
     const QueryPlan wp = plan_for<P>(qlen, g * r, db->al);
     if (scan_slices(wp.n_passes) * (size_t)wp.pass_bytes + scan_extra_smem(2, r, db->mode, ends, BLOCK) > db->smem_limit)
         f.wide_end = f.band_end;
