@@ -79,10 +79,10 @@ void *scratch_tb(hy_scratch *sc) { return sc ? sc->tb : nullptr; }
         }                                                                            \
     } while (0)
 
-template <class A, int G, int R, int MODE, bool ENDS, bool GPROF>
+template <class A, int G, int R, int MODE, bool ENDS, bool GPROF, bool ONE_COL = false>
 static cudaError_t launch_mode(const ScanParams &p, int blocks, int threads, size_t smem,
                                cudaStream_t st) {
-    auto kern = scan_kernel<A, G, R, MODE, ENDS, GPROF>;
+    auto kern = scan_kernel<A, G, R, MODE, ENDS, GPROF, ONE_COL>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -99,8 +99,24 @@ constexpr bool has_gprof_form() {
 }
 
 template <class A, int G, int R>
-static cudaError_t launch_scan(int mode, bool ends, bool gprof, const ScanParams &p, int blocks,
+static cudaError_t launch_scan(int mode, bool ends, bool gprof, bool one_col, const ScanParams &p, int blocks,
                                int threads, size_t smem, cudaStream_t st) {
+    if constexpr (A::NH == 1) {
+        if (one_col && !gprof) {
+#define HY_MODE_CASE(M)                                                                         \
+    case M:                                                                                     \
+        return ends ? launch_mode<A, G, R, M, true, false, true>(p, blocks, threads, smem, st)  \
+                    : launch_mode<A, G, R, M, false, false, true>(p, blocks, threads, smem, st);
+            switch (mode) {
+                HY_MODE_CASE(MODE_NW)
+                HY_MODE_CASE(MODE_HW)
+                HY_MODE_CASE(MODE_OV)
+                HY_MODE_CASE(MODE_SHW)
+            }
+#undef HY_MODE_CASE
+            return launch_mode<A, G, R, MODE_SW, true, false, true>(p, blocks, threads, smem, st);
+        }
+    }
     if (gprof) {
         if constexpr (has_gprof_form<A, G, R>()) {
 #define HY_MODE_CASE(M)                                                                   \
@@ -149,6 +165,37 @@ static cudaError_t launch_profile(const hy_db *db, const uint8_t *d_query, uint6
 static constexpr int32_t LIM32 = 536870911;
 static int32_t lim16(const hy_db *db) { return 32767 - db->go; }
 
+// Columns of an average item of [base, end).
+static double mean_columns(const Partition &part, uint32_t base, uint32_t end) {
+    return end > base ? (double)(part.res_prefix[end] - part.res_prefix[base]) / (end - base) : 0.0;
+}
+
+// The form of int32 items of `columns` on average: profile slices in shared or global memory, two columns a
+// step or one (the global-memory form has one).
+struct Int32Form {
+    bool gprof, one_col;
+    size_t smem;
+};
+static Int32Form int32_form(int mode, bool ends, int n_passes, size_t pass_bytes, size_t smem_limit, double columns) {
+    const size_t slices = scan_slices(n_passes) * pass_bytes;
+    const size_t two_col = slices + scan_extra_smem(1, MAIN_R32, mode, ends, BLOCK);
+    // A single pass whose slice leaves an SM one block (55 letters and up) is worth it from some 600 columns
+    // on. (60 letters, HW / SW scores: 150 columns 1.39 / 1.25 ms from global memory, 1.98 / 1.71 from shared;
+    // 400 columns 1.26 / 1.13 and 1.36 / 1.24; 1200 columns 1.41 / 1.24 and 1.25 / 1.19.)
+    const bool lone_block = n_passes == 1 && 2 * (slices + 16 + BLOCK_SMEM_RESERVE) > SM_SMEM;
+    if (slices + 16 > smem_limit || (lone_block && columns < 600)) return {true, false, 16};
+    // In the modes that look for their answer in the checked steps, of which every pass has 31 before and
+    // after the others (31 between two passes), two columns pay from some 192 columns on, 128 with more than
+    // one pass; in global mode, which has one answer, from two thirds of that. (20 letters, HW, 500 / 1,000
+    // query rows: 100 columns 1.54 / 2.99 ms with one column, 1.84 / 3.38 with two; 150 columns 1.41 / 2.72
+    // and 1.53 / 2.58; 250 columns 1.33 / 2.60 and 1.31 / 2.28.)
+    const double narrow = (mode == MODE_NW ? 128 : 192) * (n_passes > 1 ? 2 / 3.0 : 1.0);
+    // In local mode with ends the two-column sweep's copies may not fit beside slices that do (47 to 55
+    // letters): a scan_all of 20,000 targets 6.1 ms with one column, 9.4 from global memory.
+    const bool one_col = mode == MODE_SW ? two_col > smem_limit : columns < narrow;
+    return {false, one_col, one_col ? slices + 16 : two_col};
+}
+
 // Fill per-target scores (and ends) for every sequence; optionally fold the best hit key.
 // Items [item_base, item_end) of `part` (or the single item *item_ptr) on stream `st`.
 template <class A, int G, int R>
@@ -185,8 +232,15 @@ static hy_status enqueue_partition(const hy_db *db, hy_scratch *sc, const Partit
     p.wait_polls = wait_polls();
     set_extents<A>(p, db, part, part.total_cols);
     size_t smem = scan_slices(qp.n_passes) * (size_t)qp.pass_bytes + scan_extra_smem(A::NH, R, db->mode, ends, threads);
-    const bool gprof = smem > db->smem_limit;
+    bool gprof = smem > db->smem_limit, one_col = false;
     if (gprof) smem = 16;
+    if constexpr (A::NH == 1) {
+        const Int32Form f = int32_form(db->mode, ends, qp.n_passes, qp.pass_bytes, db->smem_limit,
+                                       mean_columns(part, item_base, item_end));
+        gprof = f.gprof;
+        one_col = f.one_col;
+        smem = f.smem;
+    }
     const bool timed = sc->profile && item_ptr == nullptr;
     if (timed) {
         if (sc->n_events == sc->events.size()) {
@@ -202,7 +256,7 @@ static hy_status enqueue_partition(const hy_db *db, hy_scratch *sc, const Partit
             (double)qlen * (double)(part.res_prefix[item_end] - part.res_prefix[item_base]);
         HY_CK(cudaEventRecord(sc->events[sc->n_events].first, st_));
     }
-    HY_CK((launch_scan<A, G, R>(db->mode, ends, gprof, p, blocks, threads, smem, st_)));
+    HY_CK((launch_scan<A, G, R>(db->mode, ends, gprof, one_col, p, blocks, threads, smem, st_)));
     if (timed) {
         HY_CK(cudaEventRecord(sc->events[sc->n_events].second, st_));
         ++sc->n_events;

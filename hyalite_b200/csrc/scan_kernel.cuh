@@ -1245,9 +1245,10 @@ __host__ __device__ constexpr bool scan_two_col_rows(int rows, int mode, bool en
 // for the pairs as fast as one column of 32 rows, with half the per-lane state and 10% faster on
 // 64-residue DNA queries; for the int32 items of a 5000-residue query 1014 against 594 GCUPS (two
 // independent column chains per lane for their latency-bound warps).
-template <class A, int R, int MODE, bool ENDS, bool GPROF>
+// ONE_COL: the form with one column all the same.
+template <class A, int R, int MODE, bool ENDS, bool GPROF, bool ONE_COL = false>
 __host__ __device__ constexpr bool two_col_form() {
-    return TwoCodes<A>::OK && !GPROF && scan_two_col_rows(R, MODE, ENDS);
+    return TwoCodes<A>::OK && !GPROF && !ONE_COL && scan_two_col_rows(R, MODE, ENDS);
 }
 
 #ifdef HY_BOUNDS
@@ -1300,7 +1301,7 @@ __device__ __forceinline__ void init_profile_bars(uint64_t *bars) {
 // time (the error flag is then set and the block must stop). With GPROF the lanes read the pass
 // slices straight from the profile in global memory (through L1) instead of shared memory: the
 // form for alphabets whose slices do not fit in shared memory; `smem` and `bars` are then unused.
-template <class A, int G, int R, int MODE, bool ENDS, bool GPROF = false>
+template <class A, int G, int R, int MODE, bool ENDS, bool GPROF = false, bool ONE_COL = false>
 __device__ __forceinline__ bool scan_unit(const ScanParams &p, const uint32_t item_first,
                                           const uint32_t item_end, uint8_t *smem, uint64_t *bars,
                                           uint32_t &phase) {
@@ -1341,7 +1342,7 @@ __device__ __forceinline__ bool scan_unit(const ScanParams &p, const uint32_t it
         bulk_load(smem, p.profile, p.pass_bytes, &bars[0]);
         if (p.n_passes > 1) bulk_load(smem + p.pass_bytes, p.profile + p.pass_bytes, p.pass_bytes, &bars[1]);
     }
-    if constexpr (two_col_form<A, R, MODE, ENDS, GPROF>()) {
+    if constexpr (two_col_form<A, R, MODE, ENDS, GPROF, ONE_COL>()) {
         // Column pairs a pass: at least 2G (the boundary row's read-after-write distance), and with one
         // pass the G - 1 of the fill.
         const int W = wmax == 0 ? 0 : max((int)(wmax + 1) / 2, p.n_passes > 1 ? 2 * G : G - 1);
@@ -1416,8 +1417,8 @@ inline size_t scan_extra_smem(int halves, int rows, int mode, bool ends, int thr
 // Pass slices a launch keeps in shared memory.
 __host__ __device__ inline uint32_t scan_slices(int32_t n_passes) { return n_passes > 1 ? 2 : 1; }
 
-template <class A, int G, int R, int MODE, bool ENDS, bool GPROF = false>
-__global__ void __launch_bounds__((scan_max_threads<A, G, R>()), (scan_min_blocks<A, G, R, two_col_form<A, R, MODE, ENDS, GPROF>()>()))
+template <class A, int G, int R, int MODE, bool ENDS, bool GPROF = false, bool ONE_COL = false>
+__global__ void __launch_bounds__((scan_max_threads<A, G, R>()), (scan_min_blocks<A, G, R, two_col_form<A, R, MODE, ENDS, GPROF, ONE_COL>()>()))
     scan_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (GPROF ? 0 : scan_slices(p.n_passes) * (size_t)p.pass_bytes));
@@ -1435,7 +1436,7 @@ __global__ void __launch_bounds__((scan_max_threads<A, G, R>()), (scan_min_block
     init_profile_bars(bars);
     __syncthreads();
     uint32_t phase = 0;
-    scan_unit<A, G, R, MODE, ENDS, GPROF>(p, first, end, smem, bars, phase);
+    scan_unit<A, G, R, MODE, ENDS, GPROF, ONE_COL>(p, first, end, smem, bars, phase);
 }
 
 // ---- the block-cooperative band kernel (long items, with end positions) ----------------------
