@@ -128,6 +128,7 @@ SIGNATURES = {
     "hy_debug_set_row_wait_polls": (None, [C.c_int64]),
     "hy_debug_pair_chunks": (C.c_uint64, [_u64p, _u64p, C.c_uint64, _u64p, C.c_uint64]),
     "hy_debug_pairs_idle": (C.c_int, []),
+    "hy_debug_pairs_wide_items": (C.c_uint64, []),
     "hy_debug_scan_forms": (None, [C.c_void_p, C.c_uint64, C.c_int, _u32p]),
     "hy_debug_band_plan": (_st, [C.c_int, C.c_int, C.c_uint64, C.c_uint64, C.c_uint64, _u64p]),
     "hy_debug_band_shape": (None, [C.c_uint32, C.c_int32, C.c_uint64, _i32p]),

@@ -36,6 +36,7 @@ namespace hy {
 constexpr int PAIR_G = 8;
 constexpr int PAIR_R32 = 16;
 constexpr int PAIR_WIDE_G = 32;  // lanes of the wide form: a warp an item
+constexpr size_t PAIR_SPLIT_SERIAL = 32768;  // items of a chunk whose sums one thread takes (0.09 ms)
 constexpr int PAIR_WIDE_GPB = 2;  // its items a block: small blocks, so that a long item holds little of an SM
 constexpr size_t PAIR_SMEM_LIMIT = 200 * 1024;
 // Largest global scratch for group profiles that do not fit in shared memory, per launch.
@@ -144,6 +145,7 @@ struct PairsContext {
     // staging copies, the chunk pipeline (wall time to the device's end), results, host waits for
     // a staging slot, host copies of the column maxima into the caller's array (position maxima).
     double phase_ms[7] = {0, 0, 0, 0, 0, 0, 0};
+    uint64_t wide_items = 0;  // of the last call
     ~PairsContext() {
         for (auto &x : b) hy::dev_free(x.p);
         for (auto &x : pinned) cudaFreeHost(x.p);
@@ -294,6 +296,7 @@ struct ChunkState {
     uint64_t *s_qoff, *s_toff;
     ItemMeta *s_meta[2];
     size_t n_items[2];
+    size_t n_wide;  // int16x2 items [0, n_wide) take the wide form
     uint64_t cols[2];
     uint32_t *qlen[2];
     bool narrow;  // position maxima: the chunk's column maxima go back as int16
@@ -566,11 +569,12 @@ static void sort_by_shape(PairsHost &hs, uint32_t *&o, uint64_t *&keys, uint32_t
 
 // Groups n sorted pairs into items (an int16x2 item takes two consecutive pairs of equal query
 // length) and writes their ItemMeta (columns from 0 within the chunk, each item's padded to
-// `align`) and query lengths; returns the item count and sets *cols. Boundaries come from one
+// `align`) and query lengths; returns the item count and sets *cols and, if asked, the widest item's
+// columns. Boundaries come from one
 // sequential pass over the keys; the items are filled, and their column offsets prefix-summed, on
 // all host threads.
 static size_t pack_items(PairsHost &hs, const uint32_t *order, const uint64_t *keys, size_t n,
-                         bool two, ItemMeta *meta, uint32_t *qlen, uint64_t *cols) {
+                         bool two, ItemMeta *meta, uint32_t *qlen, uint64_t *cols, uint32_t *w_max) {
     const uint64_t align = two ? 8 : 16;
     uint32_t *start = hs.start.get(n + 1);
     size_t n_items = 0;
@@ -581,10 +585,11 @@ static size_t pack_items(PairsHost &hs, const uint32_t *order, const uint64_t *k
     start[n_items] = (uint32_t)n;
     const unsigned nt = host_threads(n_items, 1 << 14);
     const uint64_t per = (n_items + nt - 1) / nt;
-    std::vector<uint64_t> part(nt + 1, 0);
+    std::vector<uint64_t> part(nt + 1, 0), widest(nt, 0);
     parallel_for(nt, 1, [&](uint64_t ta, uint64_t te, unsigned) {
         for (uint64_t t = ta; t < te; ++t) {
             uint64_t c = 0;
+            uint32_t wide = 0;
             for (uint64_t it = t * per; it < std::min<uint64_t>(n_items, (t + 1) * per); ++it) {
                 const size_t i = start[it];
                 const bool pair = start[it + 1] - i == 2;
@@ -597,9 +602,11 @@ static size_t pack_items(PairsHost &hs, const uint32_t *order, const uint64_t *k
                 m.w = std::max(m.n[0], m.n[1]);
                 m.col_off = c;  // within this thread's range; shifted below
                 c += (m.w + align - 1) / align * align;
+                wide = std::max(wide, m.w);
                 qlen[it] = key_qlen(keys[i]);
             }
             part[t + 1] = c;
+            widest[t] = wide;
         }
     });
     for (unsigned t = 0; t < nt; ++t) part[t + 1] += part[t];
@@ -609,8 +616,13 @@ static size_t pack_items(PairsHost &hs, const uint32_t *order, const uint64_t *k
                 meta[it].col_off += part[t];
     });
     *cols = part[nt];
+    if (w_max) *w_max = (uint32_t)*std::max_element(widest.begin(), widest.end());
     return n_items;
 }
+
+// Bytes a row per lane takes of a wide item's profile slice, and whether two items' slices of 8 fit a block.
+static size_t pair_wide_bytes(int32_t al) { return (size_t)(al + 1) * PAIR_WIDE_G * profile_row_bytes<Pair16H>(); }
+static bool pair_wide_fits(int32_t al) { return PAIR_WIDE_GPB * 8 * pair_wide_bytes(al) <= PAIR_SMEM_LIMIT; }
 
 // Rows per lane of the wide form: one pass of 128 rows, else passes of 256.
 static int pair_wide_rows(uint64_t q) { return q <= 128 ? 4 : 8; }
@@ -621,14 +633,25 @@ static int pair_wide_rows(uint64_t q) { return q <= 128 ? 4 : 8; }
 // least estimated time: the warp-instructions of both forms (a step of R rows 50 + 9 R) over 148 SMs of
 // 4 schedulers at 1.46 cycles, or the longest chain at 2.2. (5,000
 // protein pairs of all lengths: 6.2 ms of narrow kernels, 11.5 ms a call; so, with the long pairs' stripes
-// beside them, 5.4. 150-base reads keep the narrow form.)
-static size_t pair_wide_split(const ItemMeta *meta, const uint32_t *qlen, size_t n, int32_t al) {
+// beside them, 5.4. 150-base reads keep the narrow form.) A chunk of many short items needs no sums: where the
+// longest possible chain (the widest item, w_max columns) is shorter than what the chunk's columns take of the
+// chip, the wide form, twice the instructions a cell, gains nothing. (The sums take 2.8 ns an item, 0.3 ms of a call
+// of 200,000 read pairs where they ran on the calling thread between two chunks' staging.)
+static size_t pair_wide_split(const ItemMeta *meta, const uint32_t *qlen, size_t n, uint64_t cols, uint32_t w_max,
+                              int32_t al) {
     constexpr size_t PARTS = 16;
+    auto column = [&](uint32_t q) {  // a column of the narrow form
+        const int r = pair_rows(q, al);
+        return (double)((q + 8 * r - 1) / (8 * r)) * (50.0 + 9.0 * r);
+    };
+    const double c_max = column(qlen[0]), c_min = column(qlen[n - 1]);
+    if (std::max(c_max, c_min) * (w_max + 7.0) * 2.2 <= std::min(c_max, c_min) * (double)cols / 4 / (148 * 4) * 1.46) return 0;
     const size_t per = ((n + PARTS - 1) / PARTS + 3) / 4 * 4;  // whole warps of the narrow form
     double work[2][PARTS] = {}, chain[2][PARTS] = {};
-    uint32_t q_last = 0;
-    int r = 8;
-    for (size_t b = 0; b * per < n; ++b) {
+    auto sums = [&](size_t b) {
+        uint32_t q_last = 0;
+        int r = 8;
+        double w_narrow = 0, w_wide = 0, c_narrow = 0, c_wide = 0;
         for (size_t i = b * per; i < std::min(n, (b + 1) * per); i += 4) {
             uint32_t w = 0, q = 0;
             const size_t e = std::min(n, i + 4);
@@ -637,15 +660,22 @@ static size_t pair_wide_split(const ItemMeta *meta, const uint32_t *qlen, size_t
                 q = std::max(q, qlen[k]);
                 const int rw = pair_wide_rows(qlen[k]);
                 const double c = (double)((qlen[k] + 32 * rw - 1) / (32 * rw)) * (meta[k].w + 31.0) * (50.0 + 9.0 * rw);
-                work[1][b] += c;
-                chain[1][b] = std::max(chain[1][b], c);
+                w_wide += c;
+                c_wide = std::max(c_wide, c);
             }
             if (q != q_last) r = pair_rows(q, al), q_last = q;
             const double c = (double)((q + 8 * r - 1) / (8 * r)) * (w + 7.0) * (50.0 + 9.0 * r);
-            work[0][b] += c;
-            chain[0][b] = std::max(chain[0][b], c);
+            w_narrow += c;
+            c_narrow = std::max(c_narrow, c);
         }
-    }
+        work[0][b] = w_narrow;
+        work[1][b] = w_wide;
+        chain[0][b] = c_narrow;
+        chain[1][b] = c_wide;
+    };
+    parallel_for(PARTS, n < PAIR_SPLIT_SERIAL ? PARTS : 1, [&](uint64_t b0, uint64_t b1, unsigned) {
+        for (uint64_t b = b0; b < b1; ++b) sums(b);
+    });
     size_t best = 0;
     double best_t = 1e300;
     for (size_t s = 0; s <= PARTS; ++s) {
@@ -661,12 +691,12 @@ static size_t pair_wide_split(const ItemMeta *meta, const uint32_t *qlen, size_t
 }
 
 // Packs and aligns one chunk's items of one lane arithmetic: the packing kernel, then one launch
-// per run of items with the same rows per lane (items are sorted by query length; the wide items on
-// the side stream, joined back at the end). meta (host): the chunk's items. Items
-// [ib, ib + n_items) of the call; qlen (host) their query lengths; cols the chunk's columns.
+// per run of items with the same rows per lane (items are sorted by query length; the first n_wide, the
+// wide items, on the side stream, joined back at the end). Items [ib, ib + n_items) of the call; qlen
+// (host) their query lengths; cols the chunk's columns.
 template <class A, int G>
 static hy_status run_items(PairsContext &ctx, PairParams p, int res_slot, int bnd_slot,
-                           const uint32_t *qlen, const ItemMeta *meta, size_t ib, size_t n_items, uint64_t cols,
+                           const uint32_t *qlen, size_t n_wide, size_t ib, size_t n_items, uint64_t cols,
                            const uint64_t *d_qoff, const uint64_t *d_toff, uint8_t *d_q,
                            const uint8_t *d_t, uint32_t *d_bad, int mode, bool ends) {
     if (n_items == 0) return fail(HY_OK);
@@ -683,11 +713,6 @@ static hy_status run_items(PairsContext &ctx, PairParams p, int res_slot, int bn
     }
     // Rows per lane of each run of equal query lengths.
     auto rows_of = [&](uint32_t q) { return two ? pair_rows(q, p.al) : PAIR_R32; };
-    // The wide items [0, n_wide): not the column-maxima form, nor a large alphabet.
-    size_t n_wide = 0;
-    const size_t wide_bytes = (size_t)(p.al + 1) * PAIR_WIDE_G * profile_row_bytes<A>();  // a row per lane
-    if (two && !p.colmax && PAIR_WIDE_GPB * 8 * wide_bytes <= PAIR_SMEM_LIMIT)
-        n_wide = pair_wide_split(meta, qlen, n_items, p.al);
     bool multipass = false;
     for (size_t i = 0; i < n_wide; ++i) multipass = multipass || qlen[i] > (uint32_t)(PAIR_WIDE_G * pair_wide_rows(qlen[i]));
     for (size_t i = n_wide; i < n_items;) {
@@ -703,6 +728,7 @@ static hy_status run_items(PairsContext &ctx, PairParams p, int res_slot, int bn
     p.gprof = nullptr;
     if constexpr (two) {
         if (n_wide > 0) {
+            const size_t wide_bytes = pair_wide_bytes(p.al);
             HY_CK(cudaEventRecord(ctx.ev_fork, ctx.stream));
             HY_CK(cudaStreamWaitEvent(ctx.side_stream, ctx.ev_fork, 0));
             for (size_t i0 = 0; i0 < n_wide;) {
@@ -901,6 +927,7 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
     ctx.kernel_ms = 0.0;
     ctx.call_ms = 0.0;
     for (double &x : ctx.phase_ms) x = 0.0;
+    ctx.wide_items = 0;
     if (failed_pair) *failed_pair = n_pairs;
     if ((int)mode < 0 || (int)mode > 4) return fail(HY_ERR_INVALID_ARGUMENT);
     if ((int)search_type < HY_SEARCH_SCORE || (int)search_type > HY_SEARCH_ALIGNMENT)
@@ -1149,6 +1176,7 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             cs.s_meta[0] = (ItemMeta *)(cs.s_toff + (n + 1));
             // Every pair int16 and none on the stripe kernel: the maxima fit int16.
             cs.narrow = d_cm16 != nullptr && cnt[1] == 0 && cnt[0] == n;
+            uint32_t w_max = 0;  // columns of the widest int16x2 item
             for (int h = 0; h < 2; ++h) {
                 cs.n_items[h] = 0;
                 cs.cols[h] = 0;
@@ -1157,8 +1185,13 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
                 if (cnt[h] == 0) continue;
                 // One scratch pair serves both arithmetics: sort and pack the first before the second.
                 sort_by_shape(hs, o[h], k[h], o_tmp[h], k_tmp[h], cnt[h]);
-                cs.n_items[h] = pack_items(hs, o[h], k[h], cnt[h], h == 0, cs.s_meta[h], cs.qlen[h], &cs.cols[h]);
+                cs.n_items[h] = pack_items(hs, o[h], k[h], cnt[h], h == 0, cs.s_meta[h], cs.qlen[h], &cs.cols[h], h == 0 ? &w_max : nullptr);
             }
+            // The wide items: not of the column-maxima form, nor of a large alphabet.
+            cs.n_wide = 0;
+            if (!posmax && cs.n_items[0] && pair_wide_fits((int32_t)alphabet_len))
+                cs.n_wide = pair_wide_split(cs.s_meta[0], cs.qlen[0], cs.n_items[0], cs.cols[0], w_max, (int32_t)alphabet_len);
+            ctx.wide_items += cs.n_wide;
             parallel_for(2 * (n + 1), 1 << 18, [&](uint64_t x0, uint64_t x1, unsigned) {
                 for (uint64_t x = x0; x < x1; ++x)
                     (x <= n ? cs.s_qoff[x] : cs.s_toff[x - n - 1]) = x <= n ? q_off[a + x] : t_off[a + x - n - 1];
@@ -1187,11 +1220,11 @@ static hy_status pairs_run(const uint8_t *q_res, const uint64_t *q_off, const ui
             HY_CK(cudaStreamWaitEvent(ctx.stream, ctx.slot_ev[cs.s], 0));
             if (posmax && tb) HY_CK(cudaMemsetAsync(d_colmax + t_off[a], 0, sizeof(int32_t) * tb, ctx.stream));
             HY_CK(cudaEventRecord(ctx.ev[2 * c], ctx.stream));
-            hy_status s2 = run_items<Pair16H, PAIR_G>(ctx, pp[0], PS_RES16, PS_BND16, cs.qlen[0], cs.s_meta[0], ib[0], cs.n_items[0],
+            hy_status s2 = run_items<Pair16H, PAIR_G>(ctx, pp[0], PS_RES16, PS_BND16, cs.qlen[0], cs.n_wide, ib[0], cs.n_items[0],
                                                       cs.cols[0], (const uint64_t *)d_qoff, (const uint64_t *)d_toff,
                                                       (uint8_t *)d_q, (const uint8_t *)d_t, d_bad, mode, ends);
             if (s2 != HY_OK) return s2;
-            s2 = run_items<Single32, PAIR_G>(ctx, pp[1], PS_RES32, PS_BND32, cs.qlen[1], cs.s_meta[1], ib[1], cs.n_items[1],
+            s2 = run_items<Single32, PAIR_G>(ctx, pp[1], PS_RES32, PS_BND32, cs.qlen[1], 0, ib[1], cs.n_items[1],
                                              cs.cols[1], (const uint64_t *)d_qoff, (const uint64_t *)d_toff,
                                              (uint8_t *)d_q, (const uint8_t *)d_t, d_bad, mode, ends);
             if (s2 != HY_OK) return s2;
@@ -1425,6 +1458,9 @@ extern "C" hy_status hy_align_pairs_phases(double *ms, uint32_t n) {
     for (uint32_t i = 0; i < n && i < 7; ++i) ms[i] = g_ctx.phase_ms[i];
     return fail(HY_OK);
 }
+
+// Items of the calling thread's last align_pairs call that took the wide form.
+extern "C" uint64_t hy_debug_pairs_wide_items(void) { return g_ctx.wide_items; }
 
 // Whether the calling thread's last align_pairs call has left no work on the device.
 extern "C" int hy_debug_pairs_idle(void) { return g_ctx.idle() ? 1 : 0; }

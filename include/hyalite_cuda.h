@@ -255,6 +255,8 @@ uint64_t hy_debug_pair_chunks(const uint64_t *q_off, const uint64_t *t_off, uint
                               uint64_t *bounds, uint64_t cap);
 /* Test hook: 1 when no work of the calling thread's pairwise calls is left on the device, else 0. */
 int hy_debug_pairs_idle(void);
+/* Test hook: items of the calling thread's last hy_align_pairs call that took a warp each. */
+uint64_t hy_debug_pairs_wide_items(void);
 /* Test hook: the forms one scan of a query of qlen residues runs its items in: {int32 items, whether
  * those take the band kernel, then int16x2 pairs on the band kernel, a warp each, in the bulk kernel}. */
 void hy_debug_scan_forms(const hy_db *db, uint64_t qlen, int ends, uint32_t out[5]);
