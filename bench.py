@@ -309,24 +309,27 @@ def run_cuda(args):
         qms, ql, qc = (C.c_double * 3)(), (C.c_uint64 * 3)(), (C.c_double * 3)()
         lib.hy_scratch_profile_read(sc._h, qms, ql, qc, None)
         e = by_len.setdefault(len(queries[i]), {"queries": 0, "bulk_ms": 0.0, "bulk_cells": 0.0,
-                                                "int32_ms": 0.0, "int32_cells": 0.0, "long_ms": 0.0})
+                                                "int32_ms": 0.0, "int32_cells": 0.0, "long_ms": 0.0,
+                                                "long_cells": 0.0})
         e["queries"] += 1
         e["bulk_ms"] += qms[0]
         e["bulk_cells"] += qc[0]
         e["int32_ms"] += qms[1]
         e["int32_cells"] += qc[1]
         e["long_ms"] += qms[2]
+        e["long_cells"] += qc[2]
     lib.hy_scratch_profile(sc._h, 0)
     for e in by_len.values():
         e["bulk_gcups"] = e["bulk_cells"] / (e["bulk_ms"] * 1e-3) / 1e9 if e["bulk_ms"] > 0 else None
         e["int32_gcups"] = e["int32_cells"] / (e["int32_ms"] * 1e-3) / 1e9 if e["int32_ms"] > 0 else None
+        e["long_gcups"] = e["long_cells"] / (e["long_ms"] * 1e-3) / 1e9 if e["long_ms"] > 0 else None
 
     # ---- roofline of the dominant kernel (int16x2 pair kernel) ----
     peak = C.c_double()
     lib.hy_measure_dpx_peak(C.byref(peak))
     peak_gcups = peak.value / 1e9
     # The dominant kernel is the int16x2 pair kernel: its real cells per launch over its average
-    # launch time (CUDA events on its own stream).
+    # launch time (CUDA events on its own stream), the other forms' items beside it on the GPU.
     launches16 = max(int(kl[0]), 1)
     cells16_per_launch = kcells[0] / launches16
     avg16_ms = kms[0] / launches16
@@ -335,7 +338,9 @@ def run_cuda(args):
         return {"launches": int(kl[i]), "ms_per_step": kms[i] / args.steps, "cells_per_step": kcells[i] / args.steps,
                 "gcups": kcells[i] / (kms[i] * 1e-3) / 1e9 if kms[i] > 0 else None}
     kernels = {"bulk_int16x2_pairs": _kinfo(0), "long_int16x2_pairs": _kinfo(2), "int32_items": _kinfo(1),
-               "by_query_length_alone": {str(k): v for k, v in sorted(by_len.items())}}
+               "by_query_length_alone": {str(k): v for k, v in sorted(by_len.items())},
+               "note": "bulk pairs, pairs that left the bulk kernel (a warp each, band) and int32 items run at the "
+                       "same time on three streams: a class's rate is what it reached beside the others"}
     meas = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) if os.path.exists(
         os.path.join(ROOT, "MEASURED_PEAKS.json")) else {}
     hbm_peak = meas.get("hbm_gbs", 6650.0)

@@ -42,7 +42,8 @@ struct hy_scratch {
     // Optional event timing of the main scan kernels (hy_scratch_profile).
     bool profile = false;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> events;
-    // Kernel class of each timed launch: 0 bulk int16x2 pairs, 1 int32 items, 2 long int16x2 pairs.
+    // Kernel class of each timed launch: 0 bulk int16x2 pairs, 1 int32 items (a warp each or on the band
+    // kernel), 2 the pairs that left the bulk kernel (a warp each or on the band kernel).
     std::vector<int> event_part;
     double event_cells[3] = {0.0, 0.0, 0.0};  // real DP cells the timed launches computed
     size_t n_events = 0;
@@ -196,6 +197,27 @@ static Int32Form int32_form(int mode, bool ends, int n_passes, size_t pass_bytes
     return {false, one_col, one_col ? slices + 16 : two_col};
 }
 
+// The events around one launch of a scan's main kernels (hy_scratch_profile).
+static cudaError_t timed_begin(hy_scratch *sc, int cls, double cells, cudaStream_t st) {
+    if (sc->n_events == sc->events.size()) {
+        cudaEvent_t a, b;
+        cudaError_t e = cudaEventCreate(&a);
+        if (e == cudaSuccess) e = cudaEventCreate(&b);
+        if (e != cudaSuccess) return e;
+        sc->events.push_back({a, b});
+        sc->event_part.push_back(0);
+    }
+    sc->event_part[sc->n_events] = cls;
+    sc->event_cells[cls] += cells;
+    return cudaEventRecord(sc->events[sc->n_events].first, st);
+}
+static cudaError_t timed_end(hy_scratch *sc, cudaStream_t st) {
+    return cudaEventRecord(sc->events[sc->n_events++].second, st);
+}
+static double item_cells(const Partition &part, uint32_t base, uint32_t end, uint64_t qlen) {
+    return (double)qlen * (double)(part.res_prefix[end] - part.res_prefix[base]);
+}
+
 // Fill per-target scores (and ends) for every sequence; optionally fold the best hit key.
 // Items [item_base, item_end) of `part` (or the single item *item_ptr) on stream `st`.
 template <class A, int G, int R>
@@ -243,24 +265,11 @@ static hy_status enqueue_partition(const hy_db *db, hy_scratch *sc, const Partit
     }
     const bool timed = sc->profile && item_ptr == nullptr;
     if (timed) {
-        if (sc->n_events == sc->events.size()) {
-            cudaEvent_t a, b;
-            HY_CK(cudaEventCreate(&a));
-            HY_CK(cudaEventCreate(&b));
-            sc->events.push_back({a, b});
-            sc->event_part.push_back(0);
-        }
         const int cls = !i16 ? 1 : G == MAIN_G ? 0 : 2;
-        sc->event_part[sc->n_events] = cls;
-        sc->event_cells[cls] +=
-            (double)qlen * (double)(part.res_prefix[item_end] - part.res_prefix[item_base]);
-        HY_CK(cudaEventRecord(sc->events[sc->n_events].first, st_));
+        HY_CK(timed_begin(sc, cls, item_cells(part, item_base, item_end, qlen), st_));
     }
     HY_CK((launch_scan<A, G, R>(db->mode, ends, gprof, one_col, p, blocks, threads, smem, st_)));
-    if (timed) {
-        HY_CK(cudaEventRecord(sc->events[sc->n_events].second, st_));
-        ++sc->n_events;
-    }
+    if (timed) HY_CK(timed_end(sc, st_));
     return fail(HY_OK);
 }
 
@@ -463,7 +472,10 @@ static hy_status enqueue_band(const hy_db *db, hy_scratch *sc, const Partition &
     p.wait_polls = wait_polls();
     p.row_polls = row_wait_polls();
     set_extents<A>(p, db, part, part.total_cols);
+    const bool timed = sc->profile && item_ptr == nullptr;
+    if (timed) HY_CK(timed_begin(sc, i16 ? 2 : 1, item_cells(part, item_base, item_end, qlen), st));
     HY_CK(launch_band<A>(db->mode, sh, p, item_ptr ? 1 : item_end - item_base, st));
+    if (timed) HY_CK(timed_end(sc, st));
     sc->launches += qp.n_passes > 0 ? 2 : 1;
     return fail(HY_OK);
 }

@@ -214,9 +214,12 @@ hy_status hy_scratch_sync(hy_scratch *scratch);
 
 /* While enabled, every main scan-kernel launch on this scratch is bracketed by CUDA events on the
  * stream it runs on. _read synchronises and returns, since the last read (or enable), the summed
- * kernel time, launch count and real DP cells of the bulk int16x2 pair kernel ([0]) and the int32
- * kernel ([1]) ([2] is kept for a separate long-pair kernel, which plain scans no longer launch:
- * zero), plus the number of kernels of every kind this scratch launched; then resets them. */
+ * kernel time, launch count and real DP cells of the bulk int16x2 pair kernel ([0]), of the int32
+ * items, a warp each or on the band kernel ([1]), and of the int16x2 pairs that left the bulk
+ * kernel, a warp each or on the band kernel ([2]), plus the number of kernels of every kind this
+ * scratch launched; then resets them. Together the cells are the scan's; the three classes run at
+ * the same time on streams of their own, so a class's time is what it took beside the others, and
+ * the times do not add up to the scan's. The kernels that recover a winner's ends are not timed. */
 hy_status hy_scratch_profile(hy_scratch *scratch, int enable);
 hy_status hy_scratch_profile_read(hy_scratch *scratch, double kernel_ms[3], uint64_t launches[3],
                                   double cells[3], uint64_t *all_launches);
