@@ -1450,7 +1450,7 @@ __global__ void __launch_bounds__((scan_max_threads<A, G, R>()), (scan_min_block
 // BAND_K - 1, all written before the window's barrier since BAND_LAG >= BAND_K + 31. Between blocks
 // the last warp stores its row into the next block's ring (st.async, counted by an mbarrier per
 // BAND_K pairs there), which gives each ring block back once read; the blocks share no other step
-// (a cluster barrier a window took 2850 cycles of its 3400).
+// (no cluster barrier a window).
 //
 // A wait between blocks that gives up ends its side of that link: a block that did not get its row
 // arms and gives back no more ring blocks, one that got no space sends none from that ring block on
@@ -1460,15 +1460,15 @@ __global__ void __launch_bounds__((scan_max_threads<A, G, R>()), (scan_min_block
 // to it and that it has not read, so that no row lands in the shared memory of a block that is gone.
 //
 // What bounds it is one warp's step: a lone warp issues a chain of dependent instructions with
-// nothing beside it (one column of 4 rows a step with plain loads: 66 instructions, 250 cycles). So a
-// step has two columns whose chains are independent but for a row's lag, and as few other instructions
+// nothing beside it. So a step has two columns whose chains are independent but for a row's lag, and as few other instructions
 // as it can: residue codes lie in a strip of shared memory that is refilled every 32 steps, the row
 // above in a ring there that the warp above writes (warp 0 fills its own a window at a time, from the
 // border or from the boundary row in global memory), both read at constant offsets; a step's codes are
-// loaded two steps and its profile words one step ahead. 88 instructions, 190 cycles for two columns
-// (230 across blocks): 2000 x 2000 int32 0.47 to 0.23 ms, 5000 x 5000 1.45 to 0.67 ms. Local mode takes the short row chain (sweep_step) and tracks the best cell
-// once a step: the columns' maximum against the running one, its place looked up only where that
-// improves.
+// loaded two steps and its profile words one step ahead. 93 instructions and 258 cycles for a step of two
+// columns, over the chain of 1,751 steps of a 2000 x 2000 int32 pair on four blocks: 0.47 ms with one
+// column a step to 0.23, 5000 x 5000 1.45 to 0.67. Local mode takes the short row chain (sweep_step) and
+// tracks the best cell once a step: the columns' maximum against the running one, its place looked up
+// only where that improves.
 constexpr int BAND_K = 16;
 constexpr int BAND_LAG = 48;
 constexpr int BAND_RING = 64;  // column pairs a ring holds: at least the lag plus a window
@@ -1692,8 +1692,8 @@ __device__ __forceinline__ void band_words(const uint8_t *prof, const uint8_t *p
 // thread-block cluster: block b's warps take the passes b * W .. b * W + W - 1 of a round. `bar` is
 // an initialised mbarrier whose next wait parity is `phase` (a cluster's blocks: BAND_BARS of them,
 // not yet used); the block's dynamic shared memory (`smem`) holds W = blockDim/32 pass slices and
-// what band_smem_bytes adds. Every thread of every block must call it. With GPROF (single blocks only) the warps read their pass slices from the
-// profile in global memory; `bar` is then unused and `smem` holds the rings and strips alone.
+// what band_smem_bytes adds. Every thread of every block must call it. With GPROF (single blocks only)
+// the warps read their pass slices from the profile in global memory; `bar` is then unused and `smem` holds the rings and strips alone.
 template <class A, int R, int MODE, bool GPROF = false>
 __device__ __forceinline__ void band_item(const ScanParams &p, const uint32_t item, uint8_t *smem,
                                           uint64_t *bar, uint32_t &phase) {

@@ -809,8 +809,8 @@ static void tb_plan(uint64_t m, uint64_t max_n, uint32_t n_pairs, uint32_t *R, b
 
 // Of many pairs, the longest whose chain of passes on one warp would outlast the rest also run on
 // the stripe kernel, beside the fill: a step of R rows takes a lone warp TB_STEP_US * (R + 6), one
-// of a stripe TB_STRIPE_STEP_US, and the fill computes TB_FILL_CELLS padded cells a microsecond with
-// every SM busy (measured). A chain shorter than a third of the fill's busy time hides in it, since the
+// of a stripe TB_STRIPE_STEP_US (1.2 ms for the 3,000 of a 2000 x 2000 `align`), and the fill computes
+// TB_FILL_CELLS padded cells a microsecond with every SM busy (fitted to the call below). A chain shorter than a third of the fill's busy time hides in it, since the
 // longest pairs start first. TB_MAX_STRIPES: a stripe's warp a scheduler. (A query of 600 against 10,000
 // protein targets, 40 to some 7,000 residues: fill 8.6 to 5.6 ms.)
 constexpr double TB_STEP_US = 0.03, TB_STRIPE_STEP_US = 0.4, TB_FILL_CELLS = 775e3;
@@ -1155,8 +1155,10 @@ static hy_status tb_run(TbContext &ctx, const TbRun &run, const uint32_t *idx, u
         if (n_str > 0) {
             const cudaStream_t st = beside ? ctx.stream_s : ctx.stream;
             if (beside) {
-                // The stripes need all their blocks resident at once, so the fill, whose blocks would take
-                // the places first, waits until the stripes' stream has come as far.
+                // The stripes need all their blocks resident at once, so they should take their places before
+                // the fill's blocks do. The fill waits here only until the stripes' stream may start too; that
+                // the stripes' launch, on the stream of higher priority and issued first, is dispatched first
+                // is usual, not assured. Where it is not, they run as the fill's blocks leave: later, not wrongly.
                 TB_CK(cudaStreamWaitEvent(st, e[0], 0));
                 TB_CK(cudaEventRecord(e_str, st));
                 TB_CK(cudaStreamWaitEvent(ctx.stream, e_str, 0));
